@@ -1,0 +1,6 @@
+// The decode kernel at precision 3.
+#include "nz_decode_kernel.cuh"
+
+namespace nz {
+template int launch_decode_precision<3>(int, const BatchArgs &, uint32_t, uint32_t, cudaStream_t);
+}  // namespace nz

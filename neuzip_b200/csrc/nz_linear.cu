@@ -181,11 +181,10 @@ struct LinChain {
 };
 
 // 8 symbols of one chain as table entries (symbol in bits 23-30).
-template <int ROW>
 __device__ __forceinline__ void chain_symbols(LinChain &ch, const LutView &lv, uint32_t (&ent)[8]) {
   if (ch.kind == kUnitCoded) {
 #pragma unroll
-    for (int t = 0; t < 8; ++t) ent[t] = decode_step<ROW>(ch.st, lv);
+    for (int t = 0; t < 8; ++t) ent[t] = decode_step<kAnyRow>(ch.st, lv);
   } else {
     const uint2 q = __ldg(reinterpret_cast<const uint2 *>(ch.raw));
     ch.raw += 256;
@@ -197,8 +196,8 @@ __device__ __forceinline__ void chain_symbols(LinChain &ch, const LutView &lv, u
   }
 }
 
-template <int S, bool CANON, int ROW, bool BOTH_CODED>
-__device__ __forceinline__ bool linear_decode_loop(LinChain (&ch)[2], const LutView &lv,
+template <int S, int ROW, bool BOTH_CODED>
+__device__ __forceinline__ bool linear_decode_loop(LinChain (&ch)[2], const LutView &lv, bool canon,
                                                    uint32_t n_blocks, uint32_t stages,
                                                    uint32_t tiles0, uint32_t bar_full0,
                                                    uint32_t bar_empty0, uint32_t lane,
@@ -233,21 +232,26 @@ __device__ __forceinline__ bool linear_decode_loop(LinChain (&ch)[2], const LutV
         for (int t = 0; t < 4; ++t) {
           uint32_t e0[2], e1[2];
 #pragma unroll
-          for (int c = 0; c < 2; ++c) e0[c] = decode_step<ROW>(ch[c].st, lv);
+          for (int c = 0; c < 2; ++c) e0[c] = decode_step<ROW, usual_prob_bits(S)>(ch[c].st, lv);
 #pragma unroll
-          for (int c = 0; c < 2; ++c) e1[c] = decode_step<ROW>(ch[c].st, lv);
+          for (int c = 0; c < 2; ++c) e1[c] = decode_step<ROW, usual_prob_bits(S)>(ch[c].st, lv);
 #pragma unroll
-          for (int c = 0; c < 2; ++c) w[c][t] = merge_word<S, CANON>(e0[c], e1[c], bits[c], t);
+          for (int c = 0; c < 2; ++c) {
+            w[c][t] = merge_word<S, ROW>(e0[c], e1[c], bits[c], t);
+            if (ROW == 0 && canon) w[c][t] = canon_word(w[c][t]);
+          }
         }
       } else {
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           if (ch[c].kind == kUnitSkip) continue;
           uint32_t ent[8];
-          chain_symbols<ROW>(ch[c], lv, ent);
+          chain_symbols(ch[c], lv, ent);
 #pragma unroll
-          for (int t = 0; t < 4; ++t)
-            w[c][t] = merge_word<S, CANON>(ent[2 * t], ent[2 * t + 1], bits[c], t);
+          for (int t = 0; t < 4; ++t) {
+            w[c][t] = merge_word<S>(ent[2 * t], ent[2 * t + 1], bits[c], t);
+            if (canon) w[c][t] = canon_word(w[c][t]);
+          }
         }
       }
       // the tensor cores must be done with the tile this step overwrites
@@ -310,6 +314,10 @@ linear_kernel(const LinearArgs p, const __grid_constant__ CUtensorMap x_map) {
   a.n = (uint64_t)p.rows * p.cols;
   a.S = p.S;
   a.n_units = p.n_units;
+  a.full_units = p.n_units;            // whole row groups: no ragged unit
+  a.pay_off = payload_offset(p.n_units);
+  const uint64_t room = (p.container_bytes - a.pay_off) / 2;      // host checked: not negative
+  a.max_words = room < 0x7FFFFFFFull ? (uint32_t)room : 0x7FFFFFFFu;
   a.slot_bytes = p.slot_bytes;
   a.lut_shift = p.lut_shift;
   a.lut_bytes = p.lut_bytes;
@@ -325,6 +333,7 @@ linear_kernel(const LinearArgs p, const __grid_constant__ CUtensorMap x_map) {
   a.in = 0;
   a.seg = 0;
   a.tile_cols = p.cols;
+  a.segs = p.segs;
 
   uint8_t *misc = smem + p.lut_bytes;
   const uint32_t misc_a = base + p.lut_bytes;
@@ -372,10 +381,9 @@ linear_kernel(const LinearArgs p, const __grid_constant__ CUtensorMap x_map) {
 
   // ---- plan and stage this warp's two units, build the decode table meanwhile
   const Header *h = reinterpret_cast<const Header *>(a.container);
-  const uint64_t pay_off = payload_offset(a.n_units);
-  const uint64_t max_words = (a.container_bytes - pay_off) / 2;
   const uint32_t bar_w = misc_a + kBarWarp + 8 * (is_dec ? warp : 0);
   const uint32_t slot0 = slots_a + 2 * (is_dec ? warp : 0) * p.slot_bytes;
+  const uint4 freqs = table_prefetch(a, warp, lane);
   UnitPlan pl[2];
   uint32_t unit[2] = {p.n_units, p.n_units};
   bool staged = false;
@@ -384,11 +392,13 @@ linear_kernel(const LinearArgs p, const __grid_constant__ CUtensorMap x_map) {
     for (int c = 0; c < 2; ++c) {
       const uint32_t group = tile_id * 32 + 2 * warp + c;        // row group = 4 rows of W
       if (group < p.rows / 4) unit[c] = group * p.segs + seg;
-      pl[c] = plan_unit(a, unit[c], pay_off, max_words, lane);
+      uint32_t off0, off1;
+      unit_offsets(a, unit[c], off0, off1);
+      pl[c] = plan_unit(a, unit[c], off0, off1, lane);
     }
-    staged = stage_units(a, pl, pay_off, slot0, bar_w, lane);
+    staged = stage_units(a, pl, slot0, bar_w, lane);
   }
-  table_scan(a, h, pay_off, max_words, cum_sh, flag_sh, warp, lane, kLinWarps);
+  table_scan(a, h, freqs, cum_sh, flag_sh, warp, lane, kLinWarps);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -398,9 +408,12 @@ linear_kernel(const LinearArgs p, const __grid_constant__ CUtensorMap x_map) {
   bool ok = bad == 0;
   LutView lv;
   uint32_t row_shift = 0;
-  if (ok) table_fill(a.lut_shift, a.S, pb, smem, cum_sh, warp, lane, kLinWarps, lv, row_shift);
-  else if (threadIdx.x == 0 && blockIdx.x == 0) raise(a.status, bad);
   const bool canon = a.canon && (cum_sh[256] != cum_sh[255]);
+  // row sizes with a loop for narrow entries (see decode_kernel)
+  const uint32_t narrow_rows = canon ? 0u : (1u << 7) | (S != 7 ? 1u << 6 : 0u);
+  if (ok) table_fill(a.lut_shift, a.S, pb, smem, cum_sh, narrow_rows, usual_prob_bits(S), flag_sh, warp,
+                     lane, kLinWarps, lv, row_shift);
+  else if (threadIdx.x == 0 && blockIdx.x == 0) raise(a.status, bad);
   __syncthreads();
 
   if (is_dec) {
@@ -427,7 +440,7 @@ linear_kernel(const LinearArgs p, const __grid_constant__ CUtensorMap x_map) {
             ch[c].kind = kUnitSkip;
           }
         } else if (pl[c].kind == kUnitRaw) {
-          ch[c].raw = a.container + pay_off + pl[c].byte0 + lane * 8;
+          ch[c].raw = a.container + a.pay_off + pl[c].byte0() + lane * 8;
         }
         const uint64_t e = (uint64_t)unit[c] * U + lane * 8;        // stream order
         ch[c].frac = a.frac + e * (S + 1) / 8;
@@ -440,17 +453,17 @@ linear_kernel(const LinearArgs p, const __grid_constant__ CUtensorMap x_map) {
       const uint32_t bar_full0 = misc_a + kBarFull, bar_empty0 = misc_a + kBarEmpty;
       const bool both = ch[0].kind == kUnitCoded && ch[1].kind == kUnitCoded;
       bool fine;
-#define NZ_LIN_LOOP(CANON, ROW, BOTH)                                                          \
-  linear_decode_loop<S, CANON, ROW, BOTH>(ch, lv, n_blocks, p.stages, tiles_a, bar_full0,      \
-                                          bar_empty0, lane, abort_flag)
+#define NZ_LIN_LOOP(ROW, BOTH)                                                                 \
+  linear_decode_loop<S, ROW, BOTH>(ch, lv, canon, n_blocks, p.stages, tiles_a, bar_full0,      \
+                                   bar_empty0, lane, abort_flag)
       if (!both)
-        fine = canon ? NZ_LIN_LOOP(true, 0, false) : NZ_LIN_LOOP(false, 0, false);
-      else if (canon)
-        fine = NZ_LIN_LOOP(true, 0, true);
-      else if (row_shift == 7)
-        fine = NZ_LIN_LOOP(false, 7, true);
+        fine = NZ_LIN_LOOP(0, false);
+      else if (lv.narrow && row_shift == 7)
+        fine = NZ_LIN_LOOP(7, true);
+      else if (S != 7 && lv.narrow)
+        fine = NZ_LIN_LOOP(6, true);
       else
-        fine = NZ_LIN_LOOP(false, 0, true);
+        fine = NZ_LIN_LOOP(0, true);
 #undef NZ_LIN_LOOP
       if (!fine) {
         if (lane == 0) raise(a.status, NZ_STATUS_TIMEOUT);
