@@ -282,6 +282,13 @@ int nz_decompress_bf16_batch(const nz_decompress_item *items, uint32_t count,
                              int precision, uint32_t lane_symbols,
                              int canonical_nan, void *status, void *stream);
 
+/* nz_decompress_bf16_batch for one tensor whose description the caller keeps: `item` is
+ * only read (its out_bf16 and flags are ignored), the output and the NZ_ITEM_* flags of this
+ * call are given apart, so one description serves every read of the tensor, from any thread.
+ * Reference: Manager::read, cuda/high_level.cu:223-250. */
+int nz_decompress_bf16_item(const nz_decompress_item *item, void *out_bf16, uint32_t flags,
+                            int precision, int canonical_nan, void *status, void *stream);
+
 /* Gather: decode only the units named in `unit_ids` (a device array of n_ids
  * unit numbers, each < ceil(n / (32 * lane_symbols)); a unit is 32 *
  * lane_symbols consecutive elements) and write them one after the other:

@@ -82,6 +82,7 @@ SIGNATURES["nz_linear_vec_bf16"] = (
 SIGNATURES["nz_decompress_bf16_batch"] = (
     _int, [ctypes.POINTER(DecompressItem), _u32, _int, _u32, _int, _vp, _vp])
 
+SIGNATURES["nz_decompress_bf16_item"] = (_int, [_vp, _vp, _u32, _int, _int, _vp, _vp])
 SIGNATURES["nz_operand_lane_symbols"] = (_u32, [_u64, _int])
 SIGNATURES["nz_operand_lane_symbols_for"] = (_u32, [_u64, _u64, _int])
 SIGNATURES["nz_compress_operand_scratch_bytes"] = (_u64, [_u64, _u64, _u32])

@@ -13,6 +13,7 @@ algorithms raise ``NotImplementedError`` when constructed.
 from __future__ import annotations
 
 import enum
+import functools
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence
 
@@ -51,6 +52,9 @@ class _Entry:
     # completed the entry is settled: right-sized container, real max_unit_words.
     pending: Optional[tuple] = None
     version: int = 0          # bumped when the container tensor is replaced
+    # (argument block of a single decode, its address): struct nz_decompress_item, which the
+    # library only reads; built at the first read of these bytes
+    item: Optional[tuple] = None
 
 
 # Every operation that any backend of this process enqueues gets a number.  A decode
@@ -87,8 +91,32 @@ def _ptr(t: Optional[torch.Tensor]) -> int:
     return 0 if t is None else t.data_ptr()
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device_index = getattr(torch._C, "_cuda_getDevice", None)
+
+
 def _stream() -> int:
+    # the current stream of the current device; the raw getter is a tenth of the cost of
+    # building a torch.cuda.Stream object for it (about a microsecond per call)
+    if _raw_stream is not None and _device_index is not None and torch.cuda.is_initialized():
+        return _raw_stream(_device_index())
     return torch.cuda.current_stream().cuda_stream
+
+
+_CUDA = torch.device("cuda")         # the current device, without parsing a string per call
+
+
+@functools.lru_cache(maxsize=512)
+def _write_sizes(n: int, precision: int, lane_symbols: int):
+    """(fraction bytes, container bound, scratch bytes) of a tensor of n elements."""
+    L = _lib.load()
+    return (int(L.nz_frac_bytes(n, precision)), int(L.nz_container_bound(n, lane_symbols)),
+            int(L.nz_compress_scratch_bytes(n, lane_symbols)))
+
+
+@functools.lru_cache(maxsize=512)
+def _operand_lane_symbols(rows: int, cols: int, precision: int) -> int:
+    return int(_lib.load().nz_operand_lane_symbols_for(rows, cols, precision))
 
 
 def _require_bf16(tensor: torch.Tensor) -> None:
@@ -184,7 +212,7 @@ class CodecBackend:
         rows, cols = int(tensor.shape[0]), int(tensor.shape[1])
         if rows % 4 or cols % 64:
             return None
-        S = int(self._lib.nz_operand_lane_symbols_for(rows, cols, self.precision))
+        S = _operand_lane_symbols(rows, cols, self.precision)
         return (cols, S) if S else None
 
     def write(self, name: str, tensor: torch.Tensor, operand: Optional[bool] = None) -> None:
@@ -207,10 +235,10 @@ class CodecBackend:
         if geometry is not None:
             cols, S = geometry
             rows = n // cols
-            frac = torch.empty(int(L.nz_frac_bytes(n, self.precision)), dtype=torch.uint8, device="cuda")
-            cap = int(L.nz_container_bound(n, S))
-            staging = torch.empty(cap, dtype=torch.uint8, device="cuda")
-            scratch = self._scratch_for(int(L.nz_compress_operand_scratch_bytes(rows, cols, S)))
+            frac_bytes, cap, scratch_bytes = _write_sizes(n, self.precision, S)
+            frac = torch.empty(frac_bytes, dtype=torch.uint8, device=_CUDA)
+            staging = torch.empty(cap, dtype=torch.uint8, device=_CUDA)
+            scratch = self._scratch_for(scratch_bytes)
             _lib.check(L.nz_compress_bf16_operand(_ptr(flat), rows, cols, self.precision, S,
                                                   _ptr(frac), _ptr(staging), cap, _ptr(scratch),
                                                   scratch.numel(), st))
@@ -226,10 +254,9 @@ class CodecBackend:
             _lib.check(L.nz_normalize_bf16(_ptr(flat), n, self.normalizer_size, _ptr(scaled),
                                            _ptr(normalizers), st))
             flat = scaled
-        frac = torch.empty(int(L.nz_frac_bytes(n, self.precision)), dtype=torch.uint8, device="cuda")
-        cap = int(L.nz_container_bound(n, S))
-        staging = torch.empty(cap, dtype=torch.uint8, device="cuda")
-        scratch_bytes = int(L.nz_compress_scratch_bytes(n, S))
+        frac_bytes, cap, scratch_bytes = _write_sizes(n, self.precision, S)
+        frac = torch.empty(frac_bytes, dtype=torch.uint8, device=_CUDA)
+        staging = torch.empty(cap, dtype=torch.uint8, device=_CUDA)
         scratch = self._scratch_for(scratch_bytes)
         _lib.check(L.nz_compress_bf16(_ptr(flat), n, self.precision, S, _ptr(frac), _ptr(staging),
                                       cap, _ptr(scratch), scratch.numel(), st))
@@ -323,6 +350,7 @@ class CodecBackend:
         entry.max_unit_words = words.value
         entry.container = entry.container[:total.value].clone()     # enqueued after the write
         entry.version += 1
+        entry.item = None           # described the buffer that has just been replaced
 
     def settle_all(self) -> None:
         """Wait for every write still in flight and right-size its container (for instance
@@ -341,31 +369,51 @@ class CodecBackend:
         entry = self._get(name)
         if entry is None:
             raise RuntimeError("Data not found")
-        out = torch.empty(entry.numel, dtype=torch.bfloat16, device="cuda")
-        self.read_into(name, out)
+        out = torch.empty(entry.numel, dtype=torch.bfloat16, device=_CUDA)
+        self._decode(entry, out)
+        return out
+
+    def read_shaped(self, name: str, shape) -> torch.Tensor:
+        """`read` into a tensor of the given shape (as many elements as were written)."""
+        entry = self._get(name)
+        if entry is None:
+            raise RuntimeError("Data not found")
+        out = torch.empty(shape, dtype=torch.bfloat16, device=_CUDA)
+        if out.numel() != entry.numel:
+            raise RuntimeError(f"shape '{list(shape)}' is invalid for input of size {entry.numel}")
+        self._decode(entry, out)
         return out
 
     def read_into(self, name: str, out: torch.Tensor) -> None:
         entry = self._get(name)
         if entry is None:
             raise RuntimeError("Data not found")
-        # a batch of one: the batched entry point carries the per-item promise that the
-        # compressed bytes are not fresh, which lets this launch set up while the previous
-        # kernel of the stream drains
-        item = (_lib.DecompressItem * 1)()
-        item[0].container = _ptr(entry.container)
-        item[0].container_bytes = entry.container.numel()
-        item[0].frac_in = _ptr(entry.fractions)
-        item[0].n = entry.numel
-        item[0].max_unit_words = entry.max_unit_words
-        item[0].flags = _stable_flag([entry], _next_op())
-        item[0].out_bf16 = _ptr(out)
-        item[0].operand_cols = entry.operand_cols
-        item[0].lane_symbols = entry.lane_symbols
-        self._set_normalizer(item[0], entry)
-        _lib.check(self._lib.nz_decompress_bf16_batch(
-            item, 1, self.precision, entry.lane_symbols, int(self.canonical_nan),
-            _ptr(self._status), _stream()))
+        self._decode(entry, out)
+
+    def _decode(self, entry: _Entry, out: torch.Tensor) -> None:
+        # the per-call flag is the promise that the compressed bytes are not fresh, which lets
+        # this launch set up while the previous kernel of the stream drains
+        item = entry.item or self._describe(entry)
+        rc = self._lib.nz_decompress_bf16_item(
+            item[1], out.data_ptr(),
+            _lib.NZ_ITEM_INPUTS_STABLE if entry.stamp < _next_op() - 1 else 0,
+            self.precision, 1 if self.canonical_nan else 0, _ptr(self._status), _stream())
+        if rc:
+            _lib.check(rc)
+
+    def _describe(self, entry: _Entry):
+        """The entry's argument block for the library, filled before it is published."""
+        item = _lib.DecompressItem()
+        item.container = _ptr(entry.container)
+        item.container_bytes = entry.container.numel()
+        item.frac_in = _ptr(entry.fractions)
+        item.n = entry.numel
+        item.max_unit_words = entry.max_unit_words
+        item.operand_cols = entry.operand_cols
+        item.lane_symbols = entry.lane_symbols
+        self._set_normalizer(item, entry)
+        entry.item = described = (item, ctypes.addressof(item))
+        return described
 
     def read_rows(self, name: str, rows: torch.Tensor, row_len: int) -> torch.Tensor:
         """Rows ``rows`` (any integer tensor) of the stored tensor seen as a
@@ -379,7 +427,10 @@ class CodecBackend:
             raise RuntimeError("Data not found")
         if row_len <= 0 or entry.numel % row_len:
             raise ValueError(f"row length {row_len} does not divide the {entry.numel} stored elements")
-        rows = rows.reshape(-1).to(device="cuda", dtype=torch.int64)
+        rows = rows.reshape(-1)
+        if not (rows.is_cuda and rows.dtype == torch.int64 and rows.is_contiguous()
+                and rows.get_device() == torch.cuda.current_device()):
+            rows = rows.to(device="cuda", dtype=torch.int64).contiguous()
         k = rows.numel()
         if k == 0:
             return torch.empty(0, row_len, dtype=torch.bfloat16, device="cuda")
@@ -392,10 +443,10 @@ class CodecBackend:
         if k * per_row >= (entry.numel + U - 1) // U:
             # the lookups would decode as much as the whole table holds
             return self.read(name).view(-1, row_len)[rows]
-        out = torch.empty(k, row_len, dtype=torch.bfloat16, device="cuda")
+        out = torch.empty(k, row_len, dtype=torch.bfloat16, device=_CUDA)
         L = self._lib
         scratch_bytes = int(L.nz_gather_scratch_bytes(k, row_len, entry.lane_symbols))
-        scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device="cuda")
+        scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=_CUDA)
         _lib.check(L.nz_gather_rows_normalized_bf16(
             _ptr(entry.container), entry.container.numel(), _ptr(entry.fractions), entry.numel,
             self.precision, entry.lane_symbols, entry.max_unit_words, int(self.canonical_nan),
@@ -425,7 +476,7 @@ class CodecBackend:
             if entry is None:
                 raise RuntimeError("Data not found")
             entries.append(entry)
-        outs = [torch.empty(e.numel, dtype=torch.bfloat16, device="cuda") for e in entries]
+        outs = [torch.empty(e.numel, dtype=torch.bfloat16, device=_CUDA) for e in entries]
         # one batched call; every item names its own lane_symbols
         if entries:
             items = (_lib.DecompressItem * len(entries))()
@@ -511,24 +562,28 @@ class CodecBackend:
     def linear(self, name: str, input: torch.Tensor, shape: Sequence[int],
                bias: torch.Tensor) -> torch.Tensor:
         """cuda/high_level.cu:252-257."""
-        fused = self._linear_fused(name, input, shape, bias)
-        if fused is None:
-            fused = self._linear_vec(name, input, shape, bias)
+        fused = self._linear_while_decoding(name, input, shape, bias)
         if fused is not None:
             return fused
-        weight = self.read(name).view(*shape)
-        return torch.nn.functional.linear(input, weight, bias)
+        return torch.nn.functional.linear(input, self.read_shaped(name, shape), bias)
 
     def linear_without_bias(self, name: str, input: torch.Tensor,
                             shape: Sequence[int]) -> torch.Tensor:
         """cuda/high_level.cu:259-263."""
-        fused = self._linear_fused(name, input, shape, None)
-        if fused is None:
-            fused = self._linear_vec(name, input, shape, None)
+        fused = self._linear_while_decoding(name, input, shape, None)
         if fused is not None:
             return fused
-        weight = self.read(name).view(*shape)
-        return torch.matmul(input, weight.t())
+        return torch.nn.functional.linear(input, self.read_shaped(name, shape))
+
+    def _linear_while_decoding(self, name: str, input: torch.Tensor, shape: Sequence[int],
+                               bias: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+        """The result of whichever fused linear is switched on and takes this call, or None."""
+        fused = None
+        if self.fused_linear_max_rows:
+            fused = self._linear_fused(name, input, shape, bias)
+        if fused is None and self.fused_vector_linear:
+            fused = self._linear_vec(name, input, shape, bias)
+        return fused
 
     def linear_allreduce(self, name: str, input: torch.Tensor, shape: Sequence[int],
                          bias: Optional[torch.Tensor], reducer) -> Optional[torch.Tensor]:

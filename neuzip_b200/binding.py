@@ -90,6 +90,9 @@ class Manager:
     def read(self, handle: str) -> torch.Tensor:
         """Decompress to a CUDA tensor of the original shape (no grad)."""
         shape = self.meta_dict[handle]
+        read_shaped = getattr(self._be, "read_shaped", None)
+        if read_shaped is not None:
+            return read_shaped(handle, shape)
         return self._be.read(handle).requires_grad_(False).reshape(shape)
 
     def size(self, handle: str) -> int:

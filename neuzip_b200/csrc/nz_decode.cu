@@ -483,6 +483,19 @@ extern "C" int nz_decompress_bf16_batch(const nz_decompress_item *items, uint32_
   return NZ_OK;
 }
 
+extern "C" int nz_decompress_bf16_item(const nz_decompress_item *item, void *out_bf16, uint32_t flags,
+                                       int precision, int canonical_nan, void *status,
+                                       void *stream) {
+  if (!item) {
+    nz::set_error("nz_decompress_bf16_item: null item");
+    return NZ_E_ARG;
+  }
+  nz_decompress_item it = *item;
+  it.out_bf16 = out_bf16;
+  it.flags = flags;
+  return nz_decompress_bf16_batch(&it, 1, precision, it.lane_symbols, canonical_nan, status, stream);
+}
+
 static int decompress_units(const void *container, uint64_t container_bytes, const void *frac_in,
                             uint64_t n, int precision, uint32_t lane_symbols,
                             uint32_t max_unit_words, int canonical_nan, const void *unit_ids,

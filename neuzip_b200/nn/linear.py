@@ -68,16 +68,18 @@ class Linear(torch.nn.Module):
         return y
 
     def _forward_local(self, x):
-        if not torch.is_grad_enabled():
-            staged = self._p.staged()
+        p, bias = self._p, self.bias        # Module.__getattr__ is slow: look them up once
+        grad = torch.is_grad_enabled()
+        if not grad:
+            staged = p.staged()
             if staged is not None:          # decoded ahead for the whole block: a plain linear
-                return torch.nn.functional.linear(x, staged, self.bias)
-        if not (torch.is_grad_enabled() and (x.requires_grad or self._p.requires_grad)):
+                return torch.nn.functional.linear(x, staged, bias)
+        if not (grad and (x.requires_grad or p.requires_grad)):
             # inference: same arithmetic without the autograd.Function round trip
             if torch.is_autocast_enabled():
                 x = x.to(torch.get_autocast_gpu_dtype())
-            return self._p.linear(x, self.bias)
-        return CompressedLinear.apply(x, self._p, self.bias)
+            return p.linear(x, bias)
+        return CompressedLinear.apply(x, p, bias)
 
     # The reference's state_dict of a converted model only holds the zero-size
     # placeholder (neuzip/nn/module.py:13), so saving it loses the weights.  Here the

@@ -49,7 +49,9 @@ class Parameter(torch.nn.Parameter):
         staged = self.staged()
         if staged is not None:
             return staged
-        w = self._manager.read(self._handle).reshape(self._shape)
+        w = self._manager.read(self._handle)
+        if w.shape != self._shape:
+            w = w.reshape(self._shape)
         return w.to(self.device).requires_grad_(False)
 
     def linear_allreduce(self, inputs, bias=None):
@@ -64,4 +66,5 @@ class Parameter(torch.nn.Parameter):
         if staged is not None:
             # a layer-wise prefetch (neuzip_b200.layerwise) already decoded this weight
             return torch.nn.functional.linear(inputs, staged, bias)
-        return self._manager.linear(self._handle, inputs, bias).to(self.device)
+        y = self._manager.linear(self._handle, inputs, bias)
+        return y if y.device == self.device else y.to(self.device)
