@@ -623,7 +623,6 @@ int encode_exponents(const void *exp_in, uint64_t n, uint32_t S, void *container
 // need about 2.6).  A unit in which some lane needs more is coded again, words
 // placed straight into the slot in global memory: slower, same bytes.
 constexpr int kFusedWarps = 8;
-constexpr int kFusedChains = 1;      // units a warp codes side by side (1 or 2)
 
 template <int S>
 __device__ __forceinline__ uint32_t exp_of(uint32_t val) {
@@ -797,64 +796,94 @@ __device__ __forceinline__ void load_group(const uint16_t *__restrict__ in, uint
   }
 }
 
-// encode_step with the word going to shared memory (16-bit places from `slice`).
-__device__ __forceinline__ void encode_step_sh(uint32_t &x, int32_t &idx, uint32_t src, uint32_t sel,
-                                               uint32_t tab_addr, uint32_t slice, uint32_t pow_m) {
-  asm volatile(
-      "{\n\t"
-      ".reg .b32 s, a, xm, rc, nf, cm, q, r0, r1, j;\n\t"
-      ".reg .pred p, g;\n\t"
-      "prmt.b32 s, %2, 0, %3;\n\t"
-      "mad.lo.u32 a, s, 16, %4;\n\t"
-      "ld.shared.v4.u32 {xm, rc, nf, cm}, [a];\n\t"
-      "setp.ge.u32 p, %0, xm;\n\t"
-      "max.s32 j, %1, 1;\n\t"
-      "@p mad.lo.u32 j, j, 2, %5;\n\t"
-      "@p st.shared.u16 [j], %0;\n\t"
-      "@p shr.u32 %0, %0, 16;\n\t"
-      "@p sub.s32 %1, %1, 1;\n\t"
-      "mul.hi.u32 q, %0, rc;\n\t"
-      "mad.lo.u32 r0, q, nf, %0;\n\t"
-      "add.u32 r1, r0, nf;\n\t"
-      "setp.ge.s32 g, r1, 0;\n\t"
-      "@g add.u32 q, q, 1;\n\t"
-      "@g mov.b32 r0, r1;\n\t"
-      "add.u32 r0, r0, cm;\n\t"
-      "mad.lo.u32 %0, q, %6, r0;\n\t"
-      "}"
-      : "+r"(x), "+r"(idx)
-      : "r"(src), "r"(sel), "r"(tab_addr), "r"(slice), "r"(pow_m)
-      : "memory");
+// Encoder table of the fused kernel, 16 bytes per symbol, for x' = (x / f) * M + x % f + cum
+// with M = 2^pb written as x + bias + q * (M - f), q = x / f:
+//   x  renormalisation bound f << (32 - pb)
+//   y  reciprocal ceil(2^(32 + s) / f), with 2^s < f <= 2^(s + 1)
+//   z  bias: cum
+//   w  (M - f) << 5 | s
+// q = umulhi(x, y) >> s is exact: the reciprocal's excess makes x / f too large by less than
+// 1 / f as long as f (f - 1) < 2^(s + pb), which holds for f <= M / 2 (x < f << (32 - pb)
+// after the renormalisation).  f = 1 would need a 33-bit reciprocal; 2^32 - 1 gives q = x - 1,
+// and the bias makes up for it.  A symbol with more than half of all slots can give q one too
+// large: tensors that have one (`big`, a fact of the whole table) check the remainder.
+__device__ __forceinline__ uint4 encoder_entry(uint32_t freq, uint32_t cum, uint32_t pb) {
+  const uint32_t M = 1u << pb;
+  if (freq <= 1) return make_uint4(freq << (32 - pb), 0xFFFFFFFFu, cum + M - 1, (M - 1) << 5);
+  const uint32_t s = 31u - (uint32_t)__clz((int)(freq - 1));
+  const uint64_t num = 1ull << (32 + s);
+  return make_uint4(freq << (32 - pb), (uint32_t)((num + freq - 1) / freq), cum, ((M - freq) << 5) | s);
 }
 
-// One encoder step with the symbol's table entry already in registers: the entry only
-// depends on the symbol, so the caller fetches it a step ahead and the shared-memory
-// latency stays off the chain state -> state.  `e` = (renormalisation bound, reciprocal,
-// minus frequency, cumulative count), as bf16_encode_kernel lays the table out.
-__device__ __forceinline__ void encode_apply(uint32_t &x, int32_t &idx, const uint4 e,
-                                             uint32_t slice, uint32_t pow_m) {
-  // renormalisation without a branch: the store is predicated, shift and count are selects
-  const uint32_t full = x >= e.x;
-  const uint32_t at = slice + 2u * (uint32_t)max(idx, 1);
+// The division and update of one step, x already renormalised.
+template <bool BIG>
+__device__ __forceinline__ uint32_t encode_update(uint32_t x, const uint4 e, uint32_t pow_m) {
+  uint32_t q = __umulhi(x, e.y);
+  asm("shf.r.wrap.b32 %0, %0, 0, %1;" : "+r"(q) : "r"(e.w));      // >> s, the low 5 bits of w
+  const uint32_t cm = e.w >> 5;
+  if (BIG) {
+    const uint32_t rem = x - q * (pow_m - cm);
+    if ((int32_t)rem < 0 && cm + 1 != pow_m) --q;
+  }
+  return q * cm + (x + e.z);
+}
+
+// One step, the word going to shared memory: `pos` is the shared address of the lane's next
+// free 16-bit place and counts down.
+template <bool BIG>
+__device__ __forceinline__ void encode_step_sh(uint32_t &x, uint32_t &pos, const uint4 e,
+                                               uint32_t pow_m) {
   asm volatile(
       "{\n\t"
       ".reg .pred p;\n\t"
-      "setp.ne.u32 p, %2, 0;\n\t"
-      "@p st.shared.u16 [%0], %1;\n\t"
-      "}" ::"r"(at), "h"((uint16_t)x), "r"(full)
-      : "memory");
-  x = full ? x >> 16 : x;
-  idx -= (int32_t)full;
-  uint32_t q = __umulhi(x, e.y);
-  uint32_t r0 = q * e.z + x;                 // x - q * freq
-  const uint32_t r1 = r0 + e.z;
-  if ((int32_t)r1 >= 0) {
-    ++q;
-    r0 = r1;
-  }
-  x = q * pow_m + (r0 + e.w);
+      "setp.ge.u32 p, %0, %2;\n\t"
+      "@p st.shared.u16 [%1], %0;\n\t"
+      "@p shr.u32 %0, %0, 16;\n\t"
+      "@p add.u32 %1, %1, -2;\n\t"
+      "}"
+      : "+r"(x), "+r"(pos)
+      : "r"(e.x));
+  x = encode_update<BIG>(x, e, pow_m);
 }
 
+// Magnitudes of a pair of elements, rounded (half up) at the cut of precision S: the exponent
+// of the lower one in bits 7-14 (a carry out of it is dropped), of the upper one in 23-30, the
+// kept mantissa bits below.  Adding half a unit cannot carry from one half to the other.
+template <int S>
+__device__ __forceinline__ uint32_t round_pair(uint32_t w) {
+  const uint32_t m = w & 0x7FFF7FFFu;
+  return S < 7 ? m + 0x00010001u * (1u << (S < 7 ? 6 - S : 0)) : m;
+}
+// Packed fields of 8 elements from their words and rounded magnitudes (see split8).
+template <int S>
+__device__ __forceinline__ void pack_fields(const uint32_t (&w)[4], const uint32_t (&k)[4],
+                                            uint32_t &f0, uint32_t &f1) {
+  constexpr uint32_t kOnes = 0x00010001u;
+  uint32_t fd[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    fd[j] = ((w[j] >> (15 - S)) & ((1u << S) * kOnes)) | ((k[j] >> (7 - S)) & (((1u << S) - 1u) * kOnes));
+  f1 = 0;
+  if (S == 7) {
+    f0 = __byte_perm(fd[0], fd[1], 0x6420);
+    f1 = __byte_perm(fd[2], fd[3], 0x6420);
+  } else if (S == 3) {
+    uint32_t b[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) b[j] = ((fd[j] << 4) | (fd[j] >> 16)) & 0xFFu;
+    f0 = b[0] | (b[1] << 8) | (b[2] << 16) | (b[3] << 24);
+  } else if (S == 1) {
+    uint32_t nib[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) nib[j] = ((fd[j] & 3u) << 2) | ((fd[j] >> 16) & 3u);
+    f0 = ((nib[0] << 4) | nib[1]) | (((nib[2] << 4) | nib[3]) << 8);
+  } else {
+    uint32_t pr[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) pr[j] = ((fd[j] & 1u) << 1) | ((fd[j] >> 16) & 1u);
+    f0 = (pr[0] << 6) | (pr[1] << 4) | (pr[2] << 2) | pr[3];
+  }
+}
 
 // Second coding of a unit whose words did not fit the shared-memory slices: the
 // lengths are known from the first attempt, so every word goes straight to its
@@ -862,200 +891,194 @@ __device__ __forceinline__ void encode_apply(uint32_t &x, int32_t &idx, const ui
 template <int S>
 __device__ __noinline__ void encode_unit_in_place(const uint16_t *__restrict__ in, uint64_t n,
                                                   uint32_t LS, uint32_t cols, uint64_t first,
-                                                  uint32_t pad, uint32_t tab_addr, uint32_t pow_m,
+                                                  uint32_t pad, const uint4 *tab, uint32_t pow_m,
                                                   uint16_t *slot, uint32_t offset, uint32_t words,
                                                   uint32_t padded, uint32_t lane) {
   // the lane's stream occupies slot[offset .. offset + padded); words are emitted
   // backwards from offset + words - 1, the state ends up in the first two places
   uint16_t *mine = slot + offset;
-  int32_t idx = (int32_t)words - 1;
+  uint32_t at = words;
   uint32_t x = kStateLow;
   for (int32_t blk = (int32_t)(LS / 8) - 1; blk >= 0; --blk) {
     uint32_t lo, hi;
     load_group<S>(in, first + (uint64_t)blk * 256 + lane * 8, n, cols, pad, nullptr, false, lo, hi);
-#pragma unroll
-    for (int t = 7; t >= 0; --t)
-      encode_step(x, idx, t < 4 ? lo : hi, 0x4440u | (uint32_t)(t & 3), tab_addr, mine, pow_m);
+#pragma unroll 1
+    for (int t = 7; t >= 0; --t) {
+      const uint4 e = tab[((t < 4 ? lo : hi) >> (8 * (t & 3))) & 0xFFu];
+      if (x >= e.x) {
+        mine[--at] = (uint16_t)x;
+        x >>= 16;
+      }
+      x = encode_update<true>(x, e, pow_m);
+    }
   }
   mine[0] = (uint16_t)(x & 0xFFFFu);
   mine[1] = (uint16_t)(x >> 16);
   for (uint32_t k = words; k < padded; ++k) mine[k] = 0;
 }
 
-template <int S, int C>
+// The whole blocks of one unit, last to first.  Software pipeline: the 16 bytes of block
+// b - 2 are requested while block b is coded; the table entries are fetched two symbols ahead
+// (they depend on the symbols only), so neither latency sits on the chain state -> state.
+// A lane whose slice could run out inside a block (`limit`) starts over at its top and counts
+// what it has emitted in `spilled`: the unit is then coded a second time.
+template <int S, bool BIG>
+__device__ __forceinline__ void encode_blocks(const uint16_t *__restrict__ src, uint32_t step,
+                                              uint8_t *__restrict__ fdst, uint32_t n_blocks,
+                                              const uint8_t *tab, uint32_t pow_m, uint32_t top,
+                                              uint32_t limit, uint32_t &x, uint32_t &pos,
+                                              uint32_t &spilled) {
+  uint4 cur = __ldg(reinterpret_cast<const uint4 *>(src)), nxt = cur;
+  src -= step;
+  if (n_blocks > 1) nxt = __ldg(reinterpret_cast<const uint4 *>(src));
+#pragma unroll 1
+  for (uint32_t b = n_blocks; b > 0; --b) {
+    const uint32_t w[4] = {cur.x, cur.y, cur.z, cur.w};
+    uint32_t k[4], f0, f1;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) k[j] = round_pair<S>(w[j]);
+    // byte offset of symbol t's table entry: its exponent times 16
+    auto entry = [&](int t) {
+      const uint32_t off = (k[t >> 1] >> ((t & 1) ? 19 : 3)) & 0xFF0u;
+      return *reinterpret_cast<const uint4 *>(tab + off);
+    };
+    uint4 e0 = entry(7), e1 = entry(6);
+    cur = nxt;
+    src -= step;
+    if (b > 2) nxt = __ldg(reinterpret_cast<const uint4 *>(src));
+    pack_fields<S>(w, k, f0, f1);
+    store_fields<S>(fdst, f0, f1);
+    fdst -= 32 * (S + 1);
+    if (pos < limit) {
+      spilled += (top - pos) >> 1;
+      pos = top;
+    }
+#pragma unroll
+    for (int t = 7; t >= 0; --t) {
+      const uint4 e = e0;
+      e0 = e1;
+      if (t >= 2) e1 = entry(t - 2);
+      encode_step_sh<BIG>(x, pos, e, pow_m);
+    }
+  }
+}
+
+// What bounds it: the integer pipes (about 13 instructions per symbol, one of them a high
+// multiply that occupies its pipe four times as long) and the 16-byte table lookups (four
+// shared-memory wavefronts each).
+template <int S>
 __global__ void __launch_bounds__(kFusedWarps * 32)
 bf16_encode_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uint32_t n_units,
                    uint32_t cols, const uint32_t *__restrict__ enc_tab_g,
-                   const uint32_t *__restrict__ misc, uint32_t cap_s,
+                   const uint32_t *__restrict__ misc, uint32_t cap_s, uint32_t out_words,
                    uint8_t *__restrict__ frac_out, uint32_t *__restrict__ unit_words,
                    uint8_t *__restrict__ slots, uint32_t slot_stride) {
   extern __shared__ __align__(16) uint8_t enc_smem[];
   uint4 *tab = reinterpret_cast<uint4 *>(enc_smem);
   dependent_wait();
   const uint32_t pb = misc[1];
+  const uint32_t pow_m = 1u << pb;
+  bool over_half = false;
   for (int i = threadIdx.x; i < 256; i += blockDim.x) {
     const uint32_t e = enc_tab_g[i];
-    const uint32_t fr = e & 0xFFFFu;
-    const uint32_t rc = fr > 1 ? (uint32_t)((1ull << 32) / fr) : 0xFFFFFFFFu;
-    tab[i] = make_uint4(fr << (32 - pb), rc, 0u - fr, e >> 16);
+    tab[i] = encoder_entry(e & 0xFFFFu, e >> 16, pb);
+    over_half = over_half || (e & 0xFFFFu) > pow_m / 2;
   }
-  __syncthreads();
+  const bool big = __syncthreads_or(over_half) != 0;
   const uint32_t pad = misc[0];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t lenq = len_quantum(LS);
   const uint32_t cap = lane_cap_words(LS);
   const uint64_t U = 32ull * LS;
-  const uint32_t tab_addr = (uint32_t)__cvta_generic_to_shared(tab);
-  const uint32_t pow_m = 1u << pb;
-  // a chain's cell: 16 words of lane lengths, then 32 slices of cap_s words one word apart
+  // a warp's cell: 16 words of lane lengths, then 32 slices of cap_s words one word apart;
+  // behind it the place where the unit takes its final form
   const uint32_t sstride = cap_s + 1;
   const uint32_t cell_words = (16 + 32 * sstride + 7) & ~7u;
-  uint16_t *cell0 = reinterpret_cast<uint16_t *>(enc_smem + 4096) +
-                    (uint64_t)(warp * C) * cell_words;
+  uint16_t *cell = reinterpret_cast<uint16_t *>(enc_smem + 4096) + (uint64_t)warp * (cell_words + out_words);
+  uint16_t *unit_out = cell + cell_words;
+  const uint32_t slice = (uint32_t)__cvta_generic_to_shared(cell + 16 + lane * sstride);
+  const uint32_t top = slice + 2 * (cap_s - 1);
+  const uint32_t limit = slice + 2 * (8 + 2 - 1);      // room for a block's 8 words and the state
   const uint32_t n_warps = blockDim.x >> 5;
   const uint32_t n_blocks = LS / 8;
-  const uint32_t groups = (n_units + C - 1) / C;
-  for (uint32_t gq = blockIdx.x * n_warps + warp; gq < groups; gq += gridDim.x * n_warps) {
+  for (uint32_t u = blockIdx.x * n_warps + warp; u < n_units; u += gridDim.x * n_warps) {
     // the next kernel of the pipeline may be set up while the last units are coded
-    if (gq + gridDim.x * n_warps >= groups) dependent_trigger();
-    uint32_t u[C];
-    uint64_t first[C];
-    bool live[C];
-    uint32_t x[C], slice[C];
-    int32_t idx[C];
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-      u[c] = gq * C + c;
-      live[c] = u[c] < n_units;
-      first[c] = (uint64_t)u[c] * U;
-      x[c] = kStateLow;
-      idx[c] = (int32_t)cap_s - 1;
-      slice[c] = (uint32_t)__cvta_generic_to_shared(cell0 + c * cell_words + 16 + lane * sstride);
-    }
-    // Whole units walk two pointers down, block by block (in operand order a unit's
-    // blocks are 64 elements apart in the lane's row; otherwise 256); only the tensor's
-    // last unit can be ragged and takes the guarded loads.
-    bool whole = true;
-    const uint16_t *src[C];
-    uint8_t *fdst[C];
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-      if (live[c] && first[c] + U > n) whole = false;
-      const uint64_t e_last = first[c] + (uint64_t)(n_blocks - 1) * 256 + lane * 8;
-      src[c] = in + (live[c] && first[c] + U <= n ? source_index(e_last, cols) : 0);
-      fdst[c] = frac_out + (live[c] ? e_last * (S + 1) / 8 : 0);
-    }
-    const uint32_t step = cols ? 64u : 256u;
-    if (whole) {
-      // Software pipeline, two stages deep: the 16 bytes of block b - 2 are requested and
-      // block b - 1 is split into exponent bytes and fractions while the 8 symbols of block
-      // b are coded; inside a block, the table entry of the next symbol (of either chain)
-      // is fetched before the current one is applied.
-      uint4 nxt[C];
-      uint32_t lo[C], hi[C];
-      uint4 ent[C];
-#pragma unroll
-      for (int c = 0; c < C; ++c) {
-        uint4 cur = make_uint4(0, 0, 0, 0);
-        nxt[c] = cur;
-        if (live[c]) cur = __ldg(reinterpret_cast<const uint4 *>(src[c]));
-        src[c] -= step;
-        if (live[c] && n_blocks > 1) nxt[c] = __ldg(reinterpret_cast<const uint4 *>(src[c]));
-        const uint32_t w[4] = {cur.x, cur.y, cur.z, cur.w};
-        uint32_t f0, f1;
-        split8<S>(w, lo[c], hi[c], f0, f1);
-        if (live[c]) store_fields<S>(fdst[c], f0, f1);
-        fdst[c] -= 32 * (S + 1);
-        ent[c] = tab[hi[c] >> 24];
-      }
-      for (int32_t blk = (int32_t)n_blocks - 1; blk >= 0; --blk) {
-        // the block after this one: its bytes are here, the one after that is requested
-        uint32_t lo_n[C], hi_n[C];
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-          const uint32_t w[4] = {nxt[c].x, nxt[c].y, nxt[c].z, nxt[c].w};
-          src[c] -= step;
-          if (live[c] && blk > 1) nxt[c] = __ldg(reinterpret_cast<const uint4 *>(src[c]));
-          uint32_t f0, f1;
-          split8<S>(w, lo_n[c], hi_n[c], f0, f1);
-          if (live[c] && blk > 0) store_fields<S>(fdst[c], f0, f1);
-          fdst[c] -= 32 * (S + 1);
-        }
-#pragma unroll
-        for (int t = 7; t >= 0; --t) {
-          uint4 ahead[C];
-#pragma unroll
-          for (int c = 0; c < C; ++c) {
-            const uint32_t word = t > 4 ? hi[c] : (t > 0 ? lo[c] : hi_n[c]);   // holds symbol t - 1
-            const int byte = (t + 7) & 3;                                      // (t - 1) mod 4
-            ahead[c] = tab[(word >> (8 * byte)) & 0xFFu];
-          }
-#pragma unroll
-          for (int c = 0; c < C; ++c) encode_apply(x[c], idx[c], ent[c], slice[c], pow_m);
-#pragma unroll
-          for (int c = 0; c < C; ++c) ent[c] = ahead[c];
-        }
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-          lo[c] = lo_n[c];
-          hi[c] = hi_n[c];
-        }
-      }
+    if (u + gridDim.x * n_warps >= n_units) dependent_trigger();
+    const uint64_t first = (uint64_t)u * U;
+    const uint64_t count = (n - first < U) ? (n - first) : U;
+    uint32_t x = kStateLow, pos = top, spilled = 0;
+    if (count == U) {
+      // whole units walk two pointers down, block by block (in operand order a unit's blocks
+      // are 64 elements apart in the lane's row; otherwise 256)
+      const uint64_t e_last = first + (uint64_t)(n_blocks - 1) * 256 + lane * 8;
+      const uint16_t *src = in + source_index(e_last, cols);
+      uint8_t *fdst = frac_out + e_last * (S + 1) / 8;
+      const uint32_t step = cols ? 64u : 256u;
+      if (big)
+        encode_blocks<S, true>(src, step, fdst, n_blocks, enc_smem, pow_m, top, limit, x, pos, spilled);
+      else
+        encode_blocks<S, false>(src, step, fdst, n_blocks, enc_smem, pow_m, top, limit, x, pos, spilled);
     } else {
+      // the tensor's last unit can be ragged and takes the guarded loads
+#pragma unroll 1
       for (int32_t blk = (int32_t)n_blocks - 1; blk >= 0; --blk) {
-        uint32_t lo[C], hi[C];
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-          lo[c] = hi[c] = 0;
-          if (live[c])
-            load_group<S>(in, first[c] + (uint64_t)blk * 256 + lane * 8, n, cols, pad, frac_out,
-                          true, lo[c], hi[c]);
+        uint32_t lo, hi;
+        load_group<S>(in, first + (uint64_t)blk * 256 + lane * 8, n, cols, pad, frac_out, true, lo, hi);
+        if (pos < limit) {
+          spilled += (top - pos) >> 1;
+          pos = top;
         }
-#pragma unroll
-        for (int t = 7; t >= 0; --t) {
-#pragma unroll
-          for (int c = 0; c < C; ++c)
-            encode_step_sh(x[c], idx[c], t < 4 ? lo[c] : hi[c], 0x4440u | (uint32_t)(t & 3),
-                           tab_addr, slice[c], pow_m);
-        }
+#pragma unroll 1
+        for (int t = 7; t >= 0; --t)
+          encode_step_sh<true>(x, pos, tab[((t < 4 ? lo : hi) >> (8 * (t & 3))) & 0xFFu], pow_m);
       }
     }
+    const uint32_t words = spilled + ((top - pos) >> 1) + 2;
+    const uint32_t q = (words + lenq - 1) / lenq;
+    const uint32_t padded = q * lenq;
+    uint32_t incl = padded;
 #pragma unroll
-    for (int c = 0; c < C; ++c) {
-      if (!live[c]) continue;             // same verdict in every lane
-      uint16_t *cell = cell0 + c * cell_words;
-      const uint64_t count = (n - first[c] < U) ? (n - first[c]) : U;
-      const uint32_t emitted = (uint32_t)((int32_t)cap_s - 1 - idx[c]);
-      const uint32_t words = emitted + 2;
-      const uint32_t q = (words + lenq - 1) / lenq;
-      const uint32_t padded = q * lenq;
-      uint32_t incl = padded;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= (uint32_t)o) incl += v;
-      }
-      const uint32_t total = 16u + __shfl_sync(0xFFFFFFFFu, incl, 31);
-      const uint64_t raw_words = (count + 1) / 2;
-      const bool too_long = __any_sync(0xFFFFFFFFu, words > cap);       // the format's own limit
-      const bool raw = too_long || total >= raw_words;
-      if (lane == 0) unit_words[u[c]] = raw ? ((uint32_t)raw_words | kRawFlag) : total;
-      if (raw) continue;                  // placed from the input by place_units_kernel
-      uint16_t *slot = reinterpret_cast<uint16_t *>(slots + (uint64_t)u[c] * slot_stride);
-      if (__any_sync(0xFFFFFFFFu, words > cap_s)) {
-        // did not fit the slices: code it again, straight into the slot
-        reinterpret_cast<uint8_t *>(slot)[lane] = (uint8_t)q;
-        encode_unit_in_place<S>(in, n, LS, cols, first[c], pad, tab_addr, pow_m, slot,
-                                16 + incl - padded, words, padded, lane);
-        continue;
-      }
-      // state in front of the emitted words, then squeeze the 32 streams together
-      uint16_t *mine = cell + 16 + lane * sstride;
-      mine[cap_s - emitted - 2] = (uint16_t)(x[c] & 0xFFFFu);
-      mine[cap_s - emitted - 1] = (uint16_t)(x[c] >> 16);
-      __syncwarp();
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= (uint32_t)o) incl += v;
+    }
+    const uint32_t total = 16u + __shfl_sync(0xFFFFFFFFu, incl, 31);
+    const uint64_t raw_words = (count + 1) / 2;
+    const bool too_long = __any_sync(0xFFFFFFFFu, words > cap);       // the format's own limit
+    const bool raw = too_long || total >= raw_words;
+    if (lane == 0) unit_words[u] = raw ? ((uint32_t)raw_words | kRawFlag) : total;
+    if (raw) continue;                  // placed from the input by place_units_kernel
+    uint16_t *slot = reinterpret_cast<uint16_t *>(slots + (uint64_t)u * slot_stride);
+    if (__any_sync(0xFFFFFFFFu, spilled != 0)) {
+      // did not fit the slices: code it again, straight into the slot
+      reinterpret_cast<uint8_t *>(slot)[lane] = (uint8_t)q;
+      encode_unit_in_place<S>(in, n, LS, cols, first, pad, tab, pow_m, slot, 16 + incl - padded, words,
+                              padded, lane);
+      continue;
+    }
+    // state in front of the emitted words, then the 32 streams back to back
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(pos - 2), "r"(x) : "memory");
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(pos), "r"(x >> 16) : "memory");
+    __syncwarp();
+    const uint16_t *packed = unit_out;
+    if (total <= out_words) {
+      // every lane moves its own stream (lanes' words fall on scattered banks, two or three
+      // wavefronts a word; moving stream after stream with the whole warp cost three times
+      // the instructions)
+      reinterpret_cast<uint8_t *>(unit_out)[lane] = (uint8_t)q;
+      const uint16_t *from = cell + 16 + lane * sstride + cap_s - words;
+      uint16_t *to = unit_out + 16 + incl - padded;
+      const uint32_t longest = __reduce_max_sync(0xFFFFFFFFu, padded);
+#pragma unroll 4
+      for (uint32_t k = 0; k < longest; ++k)
+        if (k < padded) to[k] = k < words ? from[k] : (uint16_t)0;
+    } else {
+      // a unit above 3 bits per symbol: squeezed in place, stream after stream (a stream never
+      // moves up, and it ends before the next lane's slice begins)
+      packed = cell;
       reinterpret_cast<uint8_t *>(cell)[lane] = (uint8_t)q;
       uint32_t p = 16;
+#pragma unroll 1
       for (uint32_t j = 0; j < 32; ++j) {
         const uint32_t wj = __shfl_sync(0xFFFFFFFFu, words, j);
         const uint32_t pj = __shfl_sync(0xFFFFFFFFu, padded, j);
@@ -1069,12 +1092,13 @@ bf16_encode_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uin
         }
         p += pj;
       }
-      // p == total; the cell and the slot are 16-byte aligned
-      const uint4 *c4 = reinterpret_cast<const uint4 *>(cell);
-      uint4 *d4 = reinterpret_cast<uint4 *>(slot);
-      for (uint32_t k = lane; k < (total + 7) / 8; k += 32) d4[k] = c4[k];
-      __syncwarp();
     }
+    __syncwarp();
+    // cell, unit_out and slot are 16-byte aligned
+    const uint4 *c4 = reinterpret_cast<const uint4 *>(packed);
+    uint4 *d4 = reinterpret_cast<uint4 *>(slot);
+    for (uint32_t k = lane; k < (total + 7) / 8; k += 32) d4[k] = c4[k];
+    __syncwarp();
   }
 }
 
@@ -1152,7 +1176,7 @@ place_units_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uin
 
 struct FusedLayout {
   uint64_t unit_words, slots, total;
-  uint32_t slot_stride, cap_s;
+  uint32_t slot_stride, cap_s, out_words;
 };
 
 __host__ __device__ inline FusedLayout fused_layout(uint64_t n, uint32_t LS) {
@@ -1165,8 +1189,10 @@ __host__ __device__ inline FusedLayout fused_layout(uint64_t n, uint32_t LS) {
   L.slot_stride = (uint32_t)align16((16ull + 32ull * cap) * 2 + 4);
   L.slots = align16(L.unit_words + 4 * (nu + 1));
   L.total = align16(L.slots + nu * (uint64_t)L.slot_stride) + 16;
-  uint32_t cs = LS / 4 + 2;              // 4 bits per symbol and the state
-  L.cap_s = cs < cap ? cs : cap;
+  // words of a lane's slice: 4 bits per symbol, and a block's 8 words and the state of room
+  L.cap_s = LS / 4 + 10;
+  // words of a unit's final form: 3 bits per symbol (units above that are squeezed in place)
+  L.out_words = (16 + 32 * (3 * LS / 16 + 4) + 7) & ~7u;
   return L;
 }
 
@@ -1204,16 +1230,13 @@ static int compress_fused(const void *in, uint64_t n, uint32_t LS, uint32_t cols
                                low_pb));
   if (nu) {
     const uint32_t cell_words = (16 + 32 * (L.cap_s + 1) + 7) & ~7u;
-    // Units per warp: one, unless the tensor has more units than the GPU can keep resident
-    // that way -- the hardware interleaves warps better than the compiler interleaves the
-    // two chains of one warp.
-    const uint32_t chains = kFusedChains;
+    const uint32_t warp_bytes = (cell_words + L.out_words) * 2;
     // up to 8 warps per block; long lane streams get fewer so that a block still fits
-    uint32_t warps = (kMaxDynamicSmem - 4096) / (chains * cell_words * 2);
+    uint32_t warps = (kMaxDynamicSmem - 4096) / warp_bytes;
     if (warps > (uint32_t)kFusedWarps) warps = kFusedWarps;
     if (warps == 0) warps = 1;
-    const uint32_t smem = 4096 + warps * chains * cell_words * 2;
-    auto kern = bf16_encode_kernel<S, kFusedChains>;
+    const uint32_t smem = 4096 + warps * warp_bytes;
+    auto kern = bf16_encode_kernel<S>;
     {
       static std::mutex mu;
       static bool opted[kMaxDeviceOrdinals] = {};
@@ -1230,14 +1253,13 @@ static int compress_fused(const void *in, uint64_t n, uint32_t LS, uint32_t cols
       set_error("compress: lane_symbols %u needs %u bytes of shared memory per block", LS, smem);
       return NZ_E_ARG;
     }
-    const uint32_t groups = (nu + chains - 1) / chains;
-    uint32_t blocks = (groups + warps - 1) / warps;
+    uint32_t blocks = (nu + warps - 1) / warps;
     const uint32_t per_sm = kMaxDynamicSmem / (smem + 1024) ? kMaxDynamicSmem / (smem + 1024) : 1;
     const uint32_t capb = (uint32_t)sm_count() * per_sm;
     if (blocks > capb) blocks = capb;
     NZ_CUDA_TRY(launch_dependent(kern, blocks, warps * 32, smem, st, (const uint16_t *)in, n, LS, nu,
                                  cols, (const uint32_t *)(sc + kScratchTab),
-                                 (const uint32_t *)(sc + kScratchMisc), L.cap_s,
+                                 (const uint32_t *)(sc + kScratchMisc), L.cap_s, L.out_words,
                                  (uint8_t *)frac_out, (uint32_t *)(sc + L.unit_words),
                                  sc + L.slots, L.slot_stride));
   }
