@@ -12,7 +12,8 @@
 //   [0, 1024)            u32 hist[256]
 //   [1024, 1536)         u16 freq[256]
 //   [1536, 2560)         u32 enc_tab[256]   (freq | cum << 16)
-//   [2560, 2576)         u32 misc[4]        (pad symbol, probability bits, -, -)
+//   [2560, 2576)         u32 misc[4]        (pad symbol, probability bits, finished
+//                                            histogram blocks, -)
 //   [4096, 4096+4*(nu+1))           u32 unit_words[nu]  (bit 31 = raw)
 //   [.., + 64*nu)                   u16 lane_len[nu][32]   (words; 0 = unit raw)
 //   [.., + nu*32*cap*2)             u16 lane_words[nu][32][cap]   cap = lane_cap_words(S)
@@ -93,19 +94,18 @@ histogram_kernel(const uint8_t *__restrict__ sym, uint64_t n, uint32_t *__restri
 // Integer-only, identical to nzo_choose_prob_bits + nzo_normalize of the
 // specification.  The counts are 32-bit here (a tensor of 2^32 or more
 // elements is rejected by the host code), the products 64-bit.
-__global__ void normalize_kernel(const uint32_t *__restrict__ hist, uint16_t *__restrict__ freq,
-                                 uint32_t *__restrict__ enc_tab, uint32_t *__restrict__ misc,
-                                 uint16_t *__restrict__ container_freq, uint32_t low_pb) {
+// Run by one block of 256 threads.
+__device__ __forceinline__ void normalize_block(const uint32_t *hist, uint16_t *freq,
+                                                uint32_t *enc_tab, uint32_t *misc,
+                                                uint16_t *container_freq, uint32_t low_pb) {
   __shared__ int32_t f[256];
   __shared__ uint64_t red64[8];
   __shared__ uint32_t red32[8];
   __shared__ uint32_t redmx[8];
   __shared__ int32_t top_sh[8];
-  dependent_trigger();
-  dependent_wait();
   const int t = threadIdx.x;  // 256 threads
   const int lane = t & 31, wid = t >> 5;
-  const uint64_t h = hist[t];
+  const uint64_t h = __ldcg(hist + t);        // other blocks' atomics: not through L1
   // total count and number of distinct symbols
   uint64_t tot = h;
   uint32_t dis = h != 0;
@@ -225,6 +225,14 @@ __global__ void normalize_kernel(const uint32_t *__restrict__ hist, uint16_t *__
     misc[0] = (uint32_t)pad;
     misc[1] = pb;
   }
+}
+__global__ void __launch_bounds__(256)
+normalize_kernel(const uint32_t *__restrict__ hist, uint16_t *__restrict__ freq,
+                 uint32_t *__restrict__ enc_tab, uint32_t *__restrict__ misc,
+                 uint16_t *__restrict__ container_freq, uint32_t low_pb) {
+  dependent_trigger();
+  dependent_wait();
+  normalize_block(hist, freq, enc_tab, misc, container_freq, low_pb);
 }
 
 // ------------------------------------------------------------------ encoder
@@ -356,12 +364,15 @@ scan_kernel(const uint32_t *__restrict__ unit_words, uint32_t n_units, uint64_t 
   dependent_trigger();
   dependent_wait();
   const uint32_t t = threadIdx.x;
-  const uint32_t per = (n_units + 1023) / 1024;
-  const uint32_t lo = t * per < n_units ? t * per : n_units;
-  const uint32_t hi = lo + per < n_units ? lo + per : n_units;
+  // every warp has a run of consecutive units and goes over it 32 at a time, so that a warp's
+  // loads are one line (a thread with a run of its own read a line per load); first for the
+  // sums, then again for the offsets
+  const uint32_t per = ((n_units + 1023) / 1024) * 32;
+  const uint32_t lo = min((t >> 5) * per, n_units), hi = min(lo + per, n_units);
   uint64_t s = 0;
   uint32_t r = 0, m = 0;
-  for (uint32_t u = lo; u < hi; ++u) {
+#pragma unroll 4
+  for (uint32_t u = lo + (t & 31); u < hi; u += 32) {
     const uint32_t w = unit_words[u];
     s += w & ~kRawFlag;
     if (w & kRawFlag) ++r; else if (w > m) m = w;
@@ -404,7 +415,6 @@ scan_kernel(const uint32_t *__restrict__ unit_words, uint32_t n_units, uint64_t 
     }
   }
   __syncthreads();
-  const uint64_t my_start = part[wid] + incl - s;
   if (t == 0) {
     const uint64_t run = part[32];
     const uint32_t rr = raw_cnt[0], mm = max_w[0];
@@ -429,12 +439,20 @@ scan_kernel(const uint32_t *__restrict__ unit_words, uint32_t n_units, uint64_t 
     for (uint64_t b = kOffsetsOffset + 4ull * (n_units + 1); b < pay_off; ++b) container[b] = 0;
     for (uint64_t b = pay_off + run * 2; b < h.total_bytes; ++b) container[b] = 0;
   }
-  uint64_t run = my_start;
+  uint64_t run = part[wid];
   uint32_t *offsets = reinterpret_cast<uint32_t *>(container + kOffsetsOffset);
-  for (uint32_t u = lo; u < hi; ++u) {
-    const uint32_t w = unit_words[u];
-    offsets[u] = (uint32_t)run | (w & kRawFlag);
-    run += w & ~kRawFlag;
+#pragma unroll 4
+  for (uint32_t u0 = lo; u0 < hi; u0 += 32) {
+    const uint32_t u = u0 + lane;
+    const uint32_t w = u < hi ? unit_words[u] : 0u;
+    uint32_t sum = w & ~kRawFlag;            // at most 2^15 words each
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, sum, o);
+      if (lane >= (uint32_t)o) sum += v;
+    }
+    if (u < hi) offsets[u] = (uint32_t)(run + sum - (w & ~kRawFlag)) | (w & kRawFlag);
+    run += __shfl_sync(0xFFFFFFFFu, sum, 31);
   }
 }
 
@@ -632,47 +650,14 @@ __device__ __forceinline__ uint32_t exp_of(uint32_t val) {
   return (keep >> S) & 0xFFu;
 }
 
-// The 8 elements of a 16-byte load, two per 32-bit word, split with half-word
-// arithmetic: exponent bytes (lo: elements 0-3, hi: 4-7) and the S+1 bytes of packed
-// fields in memory order (f0: first four bytes, f1: the rest at precision 7).
+// Magnitudes of a pair of elements, rounded (half up) at the cut of precision S: the exponent
+// of the lower one in bits 7-14 (a carry out of it is dropped), of the upper one in 23-30, the
+// kept mantissa bits below.  Adding half a unit cannot carry from one half to the other.
 template <int S>
-__device__ __forceinline__ void split8(const uint32_t (&w)[4], uint32_t &lo, uint32_t &hi,
-                                       uint32_t &f0, uint32_t &f1) {
-  constexpr uint32_t kOnes = 0x00010001u;
-  constexpr uint32_t kKeep = ((1u << (8 + S)) - 1u) * kOnes;
-  uint32_t ex[4], fd[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const uint32_t m = w[j] & 0x7FFF7FFFu;
-    uint32_t k = (m >> (7 - S)) & kKeep;
-    if (S < 7) k = (k + ((m >> (6 - S)) & kOnes)) & kKeep;   // the carry stays inside its half
-    ex[j] = (k >> S) & 0x00FF00FFu;
-    fd[j] = ((w[j] >> (15 - S)) & ((1u << S) * kOnes)) | (k & (((1u << S) - 1u) * kOnes));
-  }
-  lo = __byte_perm(ex[0], ex[1], 0x6420);
-  hi = __byte_perm(ex[2], ex[3], 0x6420);
-  f1 = 0;
-  if (S == 7) {
-    f0 = __byte_perm(fd[0], fd[1], 0x6420);
-    f1 = __byte_perm(fd[2], fd[3], 0x6420);
-  } else if (S == 3) {
-    uint32_t b[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) b[j] = ((fd[j] << 4) | (fd[j] >> 16)) & 0xFFu;
-    f0 = b[0] | (b[1] << 8) | (b[2] << 16) | (b[3] << 24);
-  } else if (S == 1) {
-    uint32_t nib[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) nib[j] = ((fd[j] & 3u) << 2) | ((fd[j] >> 16) & 3u);
-    f0 = ((nib[0] << 4) | nib[1]) | (((nib[2] << 4) | nib[3]) << 8);
-  } else {
-    uint32_t pr[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) pr[j] = ((fd[j] & 1u) << 1) | ((fd[j] >> 16) & 1u);
-    f0 = (pr[0] << 6) | (pr[1] << 4) | (pr[2] << 2) | pr[3];
-  }
+__device__ __forceinline__ uint32_t round_pair(uint32_t w) {
+  const uint32_t m = w & 0x7FFF7FFFu;
+  return S < 7 ? m + 0x00010001u * (1u << (S < 7 ? 6 - S : 0)) : m;
 }
-
 template <int S>
 __device__ __forceinline__ void store_fields(uint8_t *dst, uint32_t f0, uint32_t f1) {
   if (S == 7) *reinterpret_cast<uint2 *>(dst) = make_uint2(f0, f1);
@@ -681,35 +666,46 @@ __device__ __forceinline__ void store_fields(uint8_t *dst, uint32_t f0, uint32_t
   else *dst = (uint8_t)f0;
 }
 
+// Exponent histogram straight from bf16, and, in the block that finishes last, the frequency
+// table made from it (a kernel of its own would add its launch to every compress).  Bound by
+// memory on large tensors: per element one shared-memory atomic and three integer
+// instructions (rounding a pair is two, a bin's address two: shift, then mask and histogram
+// base in one; the histograms are 1 KB each and aligned to it).
 template <int S>
 __global__ void __launch_bounds__(kHistThreads)
-bf16_histogram_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t *__restrict__ hist) {
-  __shared__ uint32_t sh[kHistWarps][256];
+bf16_histogram_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t *hist, uint32_t *done,
+                      uint16_t *freq, uint32_t *enc_tab, uint32_t *misc, uint16_t *container_freq,
+                      uint32_t low_pb) {
+  __shared__ __align__(1024) uint32_t sh[kHistWarps][256];
+  __shared__ uint32_t last_sh;
   dependent_wait();
   for (int i = threadIdx.x; i < kHistWarps * 256; i += kHistThreads) (&sh[0][0])[i] = 0;
   __syncthreads();
-  uint32_t *mine = sh[threadIdx.x >> 5];
+  const uint32_t mine = (uint32_t)__cvta_generic_to_shared(sh[threadIdx.x >> 5]);
+  auto count = [&](uint32_t shifted) {       // shifted: the exponent in bits 2-9
+    asm volatile("red.shared.add.u32 [%0], 1;" ::"r"((shifted & 0x3FCu) | mine) : "memory");
+  };
   const uint64_t n_vec = n / 8;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const uint4 *v = reinterpret_cast<const uint4 *>(in);
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_vec; i += stride) {
-    const uint4 q = __ldg(v + i);          // read again by the encode kernel: keep it in L2
+  auto count8 = [&](const uint4 &q) {
     const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-    uint32_t lo, hi, f0, f1;
-    split8<S>(w, lo, hi, f0, f1);
-    // one shared-memory atomic per element (a shortcut for four equal exponents in a row
-    // fires for 1.5 % of the quads of a weight matrix and costs more than it saves)
-    const uint32_t quad[2] = {lo, hi};
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      atomicAdd(&mine[quad[k] & 0xFF], 1u);
-      atomicAdd(&mine[(quad[k] >> 8) & 0xFF], 1u);
-      atomicAdd(&mine[(quad[k] >> 16) & 0xFF], 1u);
-      atomicAdd(&mine[quad[k] >> 24], 1u);
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t r = round_pair<S>(w[k]);
+      count(r >> 5);
+      count(r >> 21);
     }
+  };
+  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (; i + stride < n_vec; i += 2 * stride) {
+    const uint4 q0 = __ldg(v + i), q1 = __ldg(v + i + stride);   // read again by the encoder: kept in L2
+    count8(q0);
+    count8(q1);
   }
+  if (i < n_vec) count8(__ldg(v + i));
   if (blockIdx.x == 0 && threadIdx.x == 0)
-    for (uint64_t i = n_vec * 8; i < n; ++i) atomicAdd(&mine[exp_of<S>(in[i])], 1u);
+    for (uint64_t e = n_vec * 8; e < n; ++e) count(exp_of<S>(in[e]) << 2);
   dependent_trigger();
   __syncthreads();
   for (int b = threadIdx.x; b < 256; b += kHistThreads) {
@@ -717,6 +713,14 @@ bf16_histogram_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t *__r
 #pragma unroll
     for (int w = 0; w < kHistWarps; ++w) t += sh[w][b];
     if (t) atomicAdd(&hist[b], t);
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last_sh = atomicAdd(done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (last_sh) {
+    __threadfence();
+    normalize_block(hist, freq, enc_tab, misc, container_freq, low_pb);
   }
 }
 
@@ -846,15 +850,8 @@ __device__ __forceinline__ void encode_step_sh(uint32_t &x, uint32_t &pos, const
   x = encode_update<BIG>(x, e, pow_m);
 }
 
-// Magnitudes of a pair of elements, rounded (half up) at the cut of precision S: the exponent
-// of the lower one in bits 7-14 (a carry out of it is dropped), of the upper one in 23-30, the
-// kept mantissa bits below.  Adding half a unit cannot carry from one half to the other.
-template <int S>
-__device__ __forceinline__ uint32_t round_pair(uint32_t w) {
-  const uint32_t m = w & 0x7FFF7FFFu;
-  return S < 7 ? m + 0x00010001u * (1u << (S < 7 ? 6 - S : 0)) : m;
-}
-// Packed fields of 8 elements from their words and rounded magnitudes (see split8).
+// The S+1 bytes of packed fields of 8 elements, in memory order (f0: first four bytes, f1: the
+// rest at precision 7), from their words and rounded magnitudes.
 template <int S>
 __device__ __forceinline__ void pack_fields(const uint32_t (&w)[4], const uint32_t (&k)[4],
                                             uint32_t &f0, uint32_t &f1) {
@@ -868,10 +865,10 @@ __device__ __forceinline__ void pack_fields(const uint32_t (&w)[4], const uint32
     f0 = __byte_perm(fd[0], fd[1], 0x6420);
     f1 = __byte_perm(fd[2], fd[3], 0x6420);
   } else if (S == 3) {
-    uint32_t b[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) b[j] = ((fd[j] << 4) | (fd[j] >> 16)) & 0xFFu;
-    f0 = b[0] | (b[1] << 8) | (b[2] << 16) | (b[3] << 24);
+    // four fields in the low nibbles of four bytes; bytes 0 and 2 of p * 16 + (p >> 8) then
+    // hold a pair each
+    const uint32_t p0 = __byte_perm(fd[0], fd[1], 0x6420), p1 = __byte_perm(fd[2], fd[3], 0x6420);
+    f0 = __byte_perm(p0 * 16 + (p0 >> 8), p1 * 16 + (p1 >> 8), 0x6420);
   } else if (S == 1) {
     uint32_t nib[4];
 #pragma unroll
@@ -1129,48 +1126,38 @@ place_units_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uin
     }
     const uint32_t words = (offsets[u + 1] & ~kRawFlag) - w0;
     const uint32_t *src = reinterpret_cast<const uint32_t *>(slots + (uint64_t)u * slot_stride);
-    if ((w0 & 1) == 0) {
-      // four independent loads in flight per lane: the copy is latency-bound otherwise
-      uint32_t *d32 = reinterpret_cast<uint32_t *>(dst);
-      const uint32_t n32 = words / 2;
-      for (uint32_t k0 = 0; k0 < n32; k0 += 128) {
-        uint32_t v[4];
+    // 32-bit stores; when the destination starts on an odd word, one 16-bit store first and
+    // then source words shifted by half a word.  The copy is bound by the latency of its
+    // loads: kBatch of them are in flight per lane.
+    const uint32_t odd = w0 & 1u;
+    if (odd && lane == 0) dst[0] = reinterpret_cast<const uint16_t *>(src)[0];
+    uint32_t *d32 = reinterpret_cast<uint32_t *>(dst + odd);
+    const uint32_t pairs = (words - odd) / 2;
+    constexpr uint32_t kBatch = 12;
+    for (uint32_t k0 = 0; k0 < pairs; k0 += 32 * kBatch) {
+      uint32_t v[kBatch], after = 0;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint32_t k = k0 + 32 * i + lane;
-          v[i] = k < n32 ? __ldcs(src + k) : 0u;
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint32_t k = k0 + 32 * i + lane;
-          if (k < n32) d32[k] = v[i];
-        }
+      for (uint32_t i = 0; i < kBatch; ++i) {
+        const uint32_t k = k0 + 32 * i + lane;
+        v[i] = k < pairs + odd ? __ldcs(src + k) : 0u;
       }
-      if ((words & 1) && lane == 0)
-        dst[words - 1] = reinterpret_cast<const uint16_t *>(src)[words - 1];
-    } else {
-      // the destination starts on an odd word: one 16-bit store, then 32-bit stores of
-      // source words shifted by half a word
-      if (lane == 0) dst[0] = reinterpret_cast<const uint16_t *>(src)[0];
-      uint32_t *d32 = reinterpret_cast<uint32_t *>(dst + 1);
-      const uint32_t pairs = (words - 1) / 2;
-      for (uint32_t k0 = 0; k0 < pairs; k0 += 128) {
-        uint32_t a[4], b[4];
+      // the word after the batch, for its last lane's shift
+      if (odd && lane == 31 && k0 + 32 * kBatch < pairs + odd) after = __ldcs(src + k0 + 32 * kBatch);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint32_t k = k0 + 32 * i + lane;
-          a[i] = k < pairs ? __ldcs(src + k) : 0u;
-          b[i] = k < pairs ? __ldcs(src + k + 1) : 0u;
+      for (uint32_t i = 0; i < kBatch; ++i) {
+        const uint32_t k = k0 + 32 * i + lane;
+        uint32_t out = v[i];
+        if (odd) {
+          uint32_t next = __shfl_down_sync(0xFFFFFFFFu, v[i], 1);
+          const uint32_t first = i + 1 < kBatch ? __shfl_sync(0xFFFFFFFFu, v[i + 1 < kBatch ? i + 1 : i], 0) : after;
+          if (lane == 31) next = first;
+          out = __funnelshift_r(v[i], next, 16);
         }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint32_t k = k0 + 32 * i + lane;
-          if (k < pairs) d32[k] = __funnelshift_r(a[i], b[i], 16);
-        }
+        if (k < pairs) d32[k] = out;
       }
-      if (((words - 1) & 1) && lane == 0)
-        dst[words - 1] = reinterpret_cast<const uint16_t *>(src)[words - 1];
     }
+    if (((words - odd) & 1) && lane == 0)
+      dst[words - 1] = reinterpret_cast<const uint16_t *>(src)[words - 1];
   }
 }
 
@@ -1214,20 +1201,23 @@ static int compress_fused(const void *in, uint64_t n, uint32_t LS, uint32_t cols
   uint8_t *sc = (uint8_t *)scratch;
   uint8_t *cont = (uint8_t *)container;
   const uint32_t nu = (uint32_t)unit_count(n, LS);
-  NZ_CUDA_TRY(cudaMemsetAsync(sc + kScratchHist, 0, 1024, st));
+  // histogram, tables (overwritten) and the count of finished histogram blocks
+  NZ_CUDA_TRY(cudaMemsetAsync(sc + kScratchHist, 0, kScratchMisc + 16, st));
+  uint32_t *hist = (uint32_t *)(sc + kScratchHist), *misc = (uint32_t *)(sc + kScratchMisc);
+  uint32_t *enc_tab = (uint32_t *)(sc + kScratchTab);
+  uint16_t *freq = (uint16_t *)(sc + kScratchFreq), *cont_freq = (uint16_t *)(cont + kFreqOffset);
   if (n) {
     uint64_t blocks = (n / 8 + kHistThreads - 1) / kHistThreads;
     const uint64_t capb = (uint64_t)sm_count() * 8;
     if (blocks > capb) blocks = capb;
     if (blocks == 0) blocks = 1;
     NZ_CUDA_TRY(launch_dependent(bf16_histogram_kernel<S>, (unsigned)blocks, kHistThreads, 0, st,
-                                 (const uint16_t *)in, n, (uint32_t *)(sc + kScratchHist)));
+                                 (const uint16_t *)in, n, hist, misc + 2, freq, enc_tab, misc,
+                                 cont_freq, low_pb));
+  } else {
+    NZ_CUDA_TRY(launch_dependent(normalize_kernel, 1, 256, 0, st, (const uint32_t *)hist, freq, enc_tab,
+                                 misc, cont_freq, low_pb));
   }
-  NZ_CUDA_TRY(launch_dependent(normalize_kernel, 1, 256, 0, st,
-                               (const uint32_t *)(sc + kScratchHist),
-                               (uint16_t *)(sc + kScratchFreq), (uint32_t *)(sc + kScratchTab),
-                               (uint32_t *)(sc + kScratchMisc), (uint16_t *)(cont + kFreqOffset),
-                               low_pb));
   if (nu) {
     const uint32_t cell_words = (16 + 32 * (L.cap_s + 1) + 7) & ~7u;
     const uint32_t warp_bytes = (cell_words + L.out_words) * 2;
