@@ -12,7 +12,10 @@
 //   [0, 1024)            u32 hist[256]
 //   [1024, 1536)         u16 freq[256]
 //   [1536, 2560)         u32 enc_tab[256]   (freq | cum << 16)
-//   [2560, 2576)         u32 misc[4]        (pad symbol, probability bits, finished
+//   [2560, 2576)         u32 misc[4]        (pad symbol, probability bits, -, -)
+// and in the whole-tensor compressor
+//   [1536, 3584)         u32 entries[256][2] (reciprocal, freq | cum << 16)
+//   [3584, 3600)         u32 misc[4]        (pad symbol, probability bits, finished
 //                                            histogram blocks, -)
 //   [4096, 4096+4*(nu+1))           u32 unit_words[nu]  (bit 31 = raw)
 //   [.., + 64*nu)                   u16 lane_len[nu][32]   (words; 0 = unit raw)
@@ -29,6 +32,7 @@ constexpr uint32_t kScratchHist = 0;
 constexpr uint32_t kScratchFreq = 1024;
 constexpr uint32_t kScratchTab = 1536;
 constexpr uint32_t kScratchMisc = 2560;
+constexpr uint32_t kFusedMisc = 3584;
 constexpr uint32_t kScratchUnits = 4096;
 
 struct ScratchLayout {
@@ -94,10 +98,22 @@ histogram_kernel(const uint8_t *__restrict__ sym, uint64_t n, uint32_t *__restri
 // Integer-only, identical to nzo_choose_prob_bits + nzo_normalize of the
 // specification.  The counts are 32-bit here (a tensor of 2^32 or more
 // elements is rejected by the host code), the products 64-bit.
+// Reciprocal of a frequency for the fused encoder (see encoder_entry): ceil(2^(32 + s) / f) with
+// 2^s < f <= 2^(s + 1).
+__device__ __forceinline__ uint32_t encoder_shift(uint32_t freq) {
+  return freq > 1 ? 31u - (uint32_t)__clz((int)(freq - 1)) : 0u;
+}
+__device__ __forceinline__ uint32_t encoder_reciprocal(uint32_t freq) {
+  if (freq <= 1) return 0xFFFFFFFFu;
+  const uint64_t num = 1ull << (32 + encoder_shift(freq));
+  return (uint32_t)((num + freq - 1) / freq);
+}
+
 // Run by one block of 256 threads.
 __device__ __forceinline__ void normalize_block(const uint32_t *hist, uint16_t *freq,
-                                                uint32_t *enc_tab, uint32_t *misc,
-                                                uint16_t *container_freq, uint32_t low_pb) {
+                                                uint32_t *enc_tab, uint2 *entries,
+                                                uint32_t *misc, uint16_t *container_freq,
+                                                uint32_t low_pb) {
   __shared__ int32_t f[256];
   __shared__ uint64_t red64[8];
   __shared__ uint32_t red32[8];
@@ -217,7 +233,8 @@ __device__ __forceinline__ void normalize_block(const uint32_t *hist, uint16_t *
   for (int w = 0; w < 8; ++w)
     if (w < wid) base += top_sh[w];
   const uint32_t cum = (uint32_t)(base + incl - mine);
-  enc_tab[t] = (uint32_t)mine | (cum << 16);
+  if (enc_tab) enc_tab[t] = (uint32_t)mine | (cum << 16);
+  if (entries) entries[t] = make_uint2(encoder_reciprocal((uint32_t)mine), (uint32_t)mine | (cum << 16));
   freq[t] = (uint16_t)mine;
   container_freq[t] = (uint16_t)mine;
   const int32_t pad = block_argmax();
@@ -228,11 +245,12 @@ __device__ __forceinline__ void normalize_block(const uint32_t *hist, uint16_t *
 }
 __global__ void __launch_bounds__(256)
 normalize_kernel(const uint32_t *__restrict__ hist, uint16_t *__restrict__ freq,
-                 uint32_t *__restrict__ enc_tab, uint32_t *__restrict__ misc,
+                 uint32_t *__restrict__ enc_tab, uint2 *__restrict__ entries,
+                 uint32_t *__restrict__ misc,
                  uint16_t *__restrict__ container_freq, uint32_t low_pb) {
   dependent_trigger();
   dependent_wait();
-  normalize_block(hist, freq, enc_tab, misc, container_freq, low_pb);
+  normalize_block(hist, freq, enc_tab, entries, misc, container_freq, low_pb);
 }
 
 // ------------------------------------------------------------------ encoder
@@ -572,7 +590,7 @@ int encode_exponents(const void *exp_in, uint64_t n, uint32_t S, void *container
   if (rc) return rc;
   normalize_kernel<<<1, 256, 0, st>>>((const uint32_t *)(sc + kScratchHist),
                                       (uint16_t *)(sc + kScratchFreq),
-                                      (uint32_t *)(sc + kScratchTab),
+                                      (uint32_t *)(sc + kScratchTab), (uint2 *)nullptr,
                                       (uint32_t *)(sc + kScratchMisc),
                                       (uint16_t *)(cont + kFreqOffset), low_prob_bits);
   NZ_LAUNCH_CHECK("normalize_kernel");
@@ -626,8 +644,7 @@ int encode_exponents(const void *exp_in, uint64_t n, uint32_t S, void *container
 //      lossy precisions, exactly as the split computes them);
 //   2. bf16_encode_kernel     reads the input again (largely from L2 for tensors of
 //      the usual size), writes the packed fractions and rANS-codes the exponents.
-//      A warp codes one unit at a time (kFusedChains; two side by side measured slower:
-//      the hardware interleaves warps better than the compiler interleaves the chains of
+//      A warp codes one unit at a time (two side by side measured slower: the hardware interleaves warps better than the compiler interleaves the chains of
 //      one warp, and a warp's cells then take half the shared memory); each lane's 16-bit
 //      words go into its slice of a shared-memory cell, the
 //      cell is then squeezed into the unit's final layout and written with
@@ -672,9 +689,9 @@ __device__ __forceinline__ void store_fields(uint8_t *dst, uint32_t f0, uint32_t
 // instructions (rounding a pair is two, a bin's address two: shift, then mask and histogram
 // base in one; the histograms are 1 KB each and aligned to it).
 template <int S>
-__global__ void __launch_bounds__(kHistThreads)
+__global__ void __launch_bounds__(kHistThreads, 8)
 bf16_histogram_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t *hist, uint32_t *done,
-                      uint16_t *freq, uint32_t *enc_tab, uint32_t *misc, uint16_t *container_freq,
+                      uint16_t *freq, uint2 *entries, uint32_t *misc, uint16_t *container_freq,
                       uint32_t low_pb) {
   __shared__ __align__(1024) uint32_t sh[kHistWarps][256];
   __shared__ uint32_t last_sh;
@@ -714,13 +731,15 @@ bf16_histogram_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t *his
     for (int w = 0; w < kHistWarps; ++w) t += sh[w][b];
     if (t) atomicAdd(&hist[b], t);
   }
-  __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) last_sh = atomicAdd(done, 1u) == gridDim.x - 1;
+  if (threadIdx.x == 0) {
+    __threadfence();                 // the block's counts, ordered by the barrier, then the tally
+    last_sh = atomicAdd(done, 1u) == gridDim.x - 1;
+  }
   __syncthreads();
   if (last_sh) {
     __threadfence();
-    normalize_block(hist, freq, enc_tab, misc, container_freq, low_pb);
+    normalize_block(hist, freq, nullptr, entries, misc, container_freq, low_pb);
   }
 }
 
@@ -801,35 +820,35 @@ __device__ __forceinline__ void load_group(const uint16_t *__restrict__ in, uint
 }
 
 // Encoder table of the fused kernel, 16 bytes per symbol, for x' = (x / f) * M + x % f + cum
-// with M = 2^pb written as x + bias + q * (M - f), q = x / f:
-//   x  renormalisation bound f << (32 - pb)
-//   y  reciprocal ceil(2^(32 + s) / f), with 2^s < f <= 2^(s + 1)
-//   z  bias: cum
-//   w  (M - f) << 5 | s
-// q = umulhi(x, y) >> s is exact: the reciprocal's excess makes x / f too large by less than
-// 1 / f as long as f (f - 1) < 2^(s + pb), which holds for f <= M / 2 (x < f << (32 - pb)
-// after the renormalisation).  f = 1 would need a 33-bit reciprocal; 2^32 - 1 gives q = x - 1,
-// and the bias makes up for it.  A symbol with more than half of all slots can give q one too
-// large: tensors that have one (`big`, a fact of the whole table) check the remainder.
-__device__ __forceinline__ uint4 encoder_entry(uint32_t freq, uint32_t cum, uint32_t pb) {
-  const uint32_t M = 1u << pb;
-  if (freq <= 1) return make_uint4(freq << (32 - pb), 0xFFFFFFFFu, cum + M - 1, (M - 1) << 5);
-  const uint32_t s = 31u - (uint32_t)__clz((int)(freq - 1));
-  const uint64_t num = 1ull << (32 + s);
-  return make_uint4(freq << (32 - pb), (uint32_t)((num + freq - 1) / freq), cum, ((M - freq) << 5) | s);
+// with M = 2^pb, written as x + bias + q * (M - f), q = x / f:
+//   x  reciprocal ceil(2^(32 + s) / f), with 2^s < f <= 2^(s + 1)
+//   y  renormalisation bound f << (32 - pb)
+//   z  (M - f) << 20 | s
+//   w  bias: cum
+// q = umulhi(x, reciprocal) >> s is exact: the reciprocal's excess makes x / f too large by
+// less than 1 / f as long as f (f - 1) < 2^(s + pb), which holds for f <= M / 2 (x < f << (32 -
+// pb) after the renormalisation).  f = 1 would need a 33-bit reciprocal; 2^32 - 1 gives q = x -
+// 1, and the bias, cum + M - 1 there, makes up for it.  A symbol with more than half of all
+// slots can give q one too large: tensors that have one (`big`, a fact of the whole table)
+// check the remainder.
+constexpr uint32_t kEncTabBytes = 4096;
+__device__ __forceinline__ uint4 encoder_entry(uint2 e, uint32_t pb) {
+  const uint32_t M = 1u << pb, freq = e.y & 0xFFFFu, cum = e.y >> 16;
+  return make_uint4(e.x, freq << (32 - pb), ((M - freq) << 20) | encoder_shift(freq),
+                    freq <= 1 ? cum + M - 1 : cum);
 }
 
 // The division and update of one step, x already renormalised.
 template <bool BIG>
 __device__ __forceinline__ uint32_t encode_update(uint32_t x, const uint4 e, uint32_t pow_m) {
-  uint32_t q = __umulhi(x, e.y);
-  asm("shf.r.wrap.b32 %0, %0, 0, %1;" : "+r"(q) : "r"(e.w));      // >> s, the low 5 bits of w
-  const uint32_t cm = e.w >> 5;
+  uint32_t q = __umulhi(x, e.x);
+  asm("shf.r.wrap.b32 %0, %0, 0, %1;" : "+r"(q) : "r"(e.z));   // >> s, the low 5 bits
+  const uint32_t cm = e.z >> 20;
   if (BIG) {
     const uint32_t rem = x - q * (pow_m - cm);
-    if ((int32_t)rem < 0 && cm + 1 != pow_m) --q;
+    if ((int32_t)rem < 0) --q;
   }
-  return q * cm + (x + e.z);
+  return q * cm + (x + e.w);
 }
 
 // One step, the word going to shared memory: `pos` is the shared address of the lane's next
@@ -846,7 +865,7 @@ __device__ __forceinline__ void encode_step_sh(uint32_t &x, uint32_t &pos, const
       "@p add.u32 %1, %1, -2;\n\t"
       "}"
       : "+r"(x), "+r"(pos)
-      : "r"(e.x));
+      : "r"(e.y));
   x = encode_update<BIG>(x, e, pow_m);
 }
 
@@ -902,7 +921,7 @@ __device__ __noinline__ void encode_unit_in_place(const uint16_t *__restrict__ i
 #pragma unroll 1
     for (int t = 7; t >= 0; --t) {
       const uint4 e = tab[((t < 4 ? lo : hi) >> (8 * (t & 3))) & 0xFFu];
-      if (x >= e.x) {
+      if (x >= e.y) {
         mine[--at] = (uint16_t)x;
         x >>= 16;
       }
@@ -922,7 +941,7 @@ __device__ __noinline__ void encode_unit_in_place(const uint16_t *__restrict__ i
 template <int S, bool BIG>
 __device__ __forceinline__ void encode_blocks(const uint16_t *__restrict__ src, uint32_t step,
                                               uint8_t *__restrict__ fdst, uint32_t n_blocks,
-                                              const uint8_t *tab, uint32_t pow_m, uint32_t top,
+                                              const uint4 *tab, uint32_t pow_m, uint32_t top,
                                               uint32_t limit, uint32_t &x, uint32_t &pos,
                                               uint32_t &spilled) {
   uint4 cur = __ldg(reinterpret_cast<const uint4 *>(src)), nxt = cur;
@@ -934,10 +953,10 @@ __device__ __forceinline__ void encode_blocks(const uint16_t *__restrict__ src, 
     uint32_t k[4], f0, f1;
 #pragma unroll
     for (int j = 0; j < 4; ++j) k[j] = round_pair<S>(w[j]);
-    // byte offset of symbol t's table entry: its exponent times 16
+    // symbol t's table entry: byte offset 16 times its exponent
     auto entry = [&](int t) {
       const uint32_t off = (k[t >> 1] >> ((t & 1) ? 19 : 3)) & 0xFF0u;
-      return *reinterpret_cast<const uint4 *>(tab + off);
+      return *reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(tab) + off);
     };
     uint4 e0 = entry(7), e1 = entry(6);
     cur = nxt;
@@ -966,7 +985,7 @@ __device__ __forceinline__ void encode_blocks(const uint16_t *__restrict__ src, 
 template <int S>
 __global__ void __launch_bounds__(kFusedWarps * 32)
 bf16_encode_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uint32_t n_units,
-                   uint32_t cols, const uint32_t *__restrict__ enc_tab_g,
+                   uint32_t cols, const uint2 *__restrict__ entries,
                    const uint32_t *__restrict__ misc, uint32_t cap_s, uint32_t out_words,
                    uint8_t *__restrict__ frac_out, uint32_t *__restrict__ unit_words,
                    uint8_t *__restrict__ slots, uint32_t slot_stride) {
@@ -977,9 +996,9 @@ bf16_encode_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uin
   const uint32_t pow_m = 1u << pb;
   bool over_half = false;
   for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-    const uint32_t e = enc_tab_g[i];
-    tab[i] = encoder_entry(e & 0xFFFFu, e >> 16, pb);
-    over_half = over_half || (e & 0xFFFFu) > pow_m / 2;
+    const uint2 e = entries[i];
+    tab[i] = encoder_entry(e, pb);
+    over_half = over_half || (e.y & 0xFFFFu) > pow_m / 2;
   }
   const bool big = __syncthreads_or(over_half) != 0;
   const uint32_t pad = misc[0];
@@ -991,7 +1010,8 @@ bf16_encode_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uin
   // behind it the place where the unit takes its final form
   const uint32_t sstride = cap_s + 1;
   const uint32_t cell_words = (16 + 32 * sstride + 7) & ~7u;
-  uint16_t *cell = reinterpret_cast<uint16_t *>(enc_smem + 4096) + (uint64_t)warp * (cell_words + out_words);
+  uint16_t *cell = reinterpret_cast<uint16_t *>(enc_smem + kEncTabBytes) +
+                   (uint64_t)warp * (cell_words + out_words);
   uint16_t *unit_out = cell + cell_words;
   const uint32_t slice = (uint32_t)__cvta_generic_to_shared(cell + 16 + lane * sstride);
   const uint32_t top = slice + 2 * (cap_s - 1);
@@ -1012,9 +1032,9 @@ bf16_encode_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uin
       uint8_t *fdst = frac_out + e_last * (S + 1) / 8;
       const uint32_t step = cols ? 64u : 256u;
       if (big)
-        encode_blocks<S, true>(src, step, fdst, n_blocks, enc_smem, pow_m, top, limit, x, pos, spilled);
+        encode_blocks<S, true>(src, step, fdst, n_blocks, tab, pow_m, top, limit, x, pos, spilled);
       else
-        encode_blocks<S, false>(src, step, fdst, n_blocks, enc_smem, pow_m, top, limit, x, pos, spilled);
+        encode_blocks<S, false>(src, step, fdst, n_blocks, tab, pow_m, top, limit, x, pos, spilled);
     } else {
       // the tensor's last unit can be ragged and takes the guarded loads
 #pragma unroll 1
@@ -1058,17 +1078,31 @@ bf16_encode_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uin
     asm volatile("st.shared.u16 [%0], %1;" ::"r"(pos), "r"(x >> 16) : "memory");
     __syncwarp();
     const uint16_t *packed = unit_out;
-    if (total <= out_words) {
-      // every lane moves its own stream (lanes' words fall on scattered banks, two or three
-      // wavefronts a word; moving stream after stream with the whole warp cost three times
-      // the instructions)
+    if (lenq == 1 && total <= out_words) {
+      // every lane moves its own stream, 32 bits at a time (lanes' words fall on scattered
+      // banks, two or three wavefronts each; moving stream after stream with the whole warp
+      // cost three times the instructions).  Words j of the destination take halves of source
+      // words base + j and base + j + 1; a half word at either end is stored by itself.
       reinterpret_cast<uint8_t *>(unit_out)[lane] = (uint8_t)q;
-      const uint16_t *from = cell + 16 + lane * sstride + cap_s - words;
-      uint16_t *to = unit_out + 16 + incl - padded;
-      const uint32_t longest = __reduce_max_sync(0xFFFFFFFFu, padded);
+      const uint32_t from = 16 + lane * sstride + cap_s - words, to = 16 + incl - padded;
+      const uint32_t odd = to & 1u, base = (from - odd) >> 1, shift = ((from - odd) & 1u) * 16u;
+      const uint32_t *src32 = reinterpret_cast<const uint32_t *>(cell) + base;
+      uint32_t *dst32 = reinterpret_cast<uint32_t *>(unit_out) + (to >> 1);
+      const uint32_t full = ((to + words) >> 1) - (to >> 1);     // destination words that end inside
+      const uint32_t longest = __reduce_max_sync(0xFFFFFFFFu, full);
+      uint32_t here = src32[0];
 #pragma unroll 4
-      for (uint32_t k = 0; k < longest; ++k)
-        if (k < padded) to[k] = k < words ? from[k] : (uint16_t)0;
+      for (uint32_t j = 0; j < longest; ++j) {
+        if (j < full) {
+          const uint32_t next = src32[j + 1];
+          const uint32_t v = __funnelshift_r(here, next, shift);
+          if (j || !odd) dst32[j] = v;
+          else reinterpret_cast<uint16_t *>(dst32)[1] = (uint16_t)(v >> 16);
+          here = next;
+        }
+      }
+      if ((to + words) & 1u)
+        unit_out[to + words - 1] = cell[from + words - 1];
     } else {
       // a unit above 3 bits per symbol: squeezed in place, stream after stream (a stream never
       // moves up, and it ends before the next lane's slice begins)
@@ -1202,9 +1236,9 @@ static int compress_fused(const void *in, uint64_t n, uint32_t LS, uint32_t cols
   uint8_t *cont = (uint8_t *)container;
   const uint32_t nu = (uint32_t)unit_count(n, LS);
   // histogram, tables (overwritten) and the count of finished histogram blocks
-  NZ_CUDA_TRY(cudaMemsetAsync(sc + kScratchHist, 0, kScratchMisc + 16, st));
-  uint32_t *hist = (uint32_t *)(sc + kScratchHist), *misc = (uint32_t *)(sc + kScratchMisc);
-  uint32_t *enc_tab = (uint32_t *)(sc + kScratchTab);
+  NZ_CUDA_TRY(cudaMemsetAsync(sc + kScratchHist, 0, kFusedMisc + 16, st));
+  uint32_t *hist = (uint32_t *)(sc + kScratchHist), *misc = (uint32_t *)(sc + kFusedMisc);
+  uint2 *entries = (uint2 *)(sc + kScratchTab);
   uint16_t *freq = (uint16_t *)(sc + kScratchFreq), *cont_freq = (uint16_t *)(cont + kFreqOffset);
   if (n) {
     uint64_t blocks = (n / 8 + kHistThreads - 1) / kHistThreads;
@@ -1212,20 +1246,20 @@ static int compress_fused(const void *in, uint64_t n, uint32_t LS, uint32_t cols
     if (blocks > capb) blocks = capb;
     if (blocks == 0) blocks = 1;
     NZ_CUDA_TRY(launch_dependent(bf16_histogram_kernel<S>, (unsigned)blocks, kHistThreads, 0, st,
-                                 (const uint16_t *)in, n, hist, misc + 2, freq, enc_tab, misc,
+                                 (const uint16_t *)in, n, hist, misc + 2, freq, entries, misc,
                                  cont_freq, low_pb));
   } else {
-    NZ_CUDA_TRY(launch_dependent(normalize_kernel, 1, 256, 0, st, (const uint32_t *)hist, freq, enc_tab,
-                                 misc, cont_freq, low_pb));
+    NZ_CUDA_TRY(launch_dependent(normalize_kernel, 1, 256, 0, st, (const uint32_t *)hist, freq,
+                                 (uint32_t *)nullptr, entries, misc, cont_freq, low_pb));
   }
   if (nu) {
     const uint32_t cell_words = (16 + 32 * (L.cap_s + 1) + 7) & ~7u;
     const uint32_t warp_bytes = (cell_words + L.out_words) * 2;
-    // up to 8 warps per block; long lane streams get fewer so that a block still fits
-    uint32_t warps = (kMaxDynamicSmem - 4096) / warp_bytes;
+    // up to kFusedWarps per block; long lane streams get fewer so that a block still fits
+    uint32_t warps = (kMaxDynamicSmem - kEncTabBytes) / warp_bytes;
     if (warps > (uint32_t)kFusedWarps) warps = kFusedWarps;
     if (warps == 0) warps = 1;
-    const uint32_t smem = 4096 + warps * warp_bytes;
+    const uint32_t smem = kEncTabBytes + warps * warp_bytes;
     auto kern = bf16_encode_kernel<S>;
     {
       static std::mutex mu;
@@ -1248,13 +1282,12 @@ static int compress_fused(const void *in, uint64_t n, uint32_t LS, uint32_t cols
     const uint32_t capb = (uint32_t)sm_count() * per_sm;
     if (blocks > capb) blocks = capb;
     NZ_CUDA_TRY(launch_dependent(kern, blocks, warps * 32, smem, st, (const uint16_t *)in, n, LS, nu,
-                                 cols, (const uint32_t *)(sc + kScratchTab),
-                                 (const uint32_t *)(sc + kScratchMisc), L.cap_s, L.out_words,
+                                 cols, (const uint2 *)entries, (const uint32_t *)misc, L.cap_s, L.out_words,
                                  (uint8_t *)frac_out, (uint32_t *)(sc + L.unit_words),
                                  sc + L.slots, L.slot_stride));
   }
   NZ_CUDA_TRY(launch_dependent(scan_kernel, 1, 1024, 0, st, (const uint32_t *)(sc + L.unit_words),
-                               nu, n, LS, (const uint32_t *)(sc + kScratchMisc), cont));
+                               nu, n, LS, (const uint32_t *)misc, cont));
   if (nu) {
     uint32_t blocks = (nu + 3) / 4;
     const uint32_t capb = (uint32_t)sm_count() * 16;

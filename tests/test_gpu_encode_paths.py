@@ -1,0 +1,50 @@
+"""Branches of the fused encoder, each against the oracle byte for byte: a symbol with more
+than half of the slots (the remainder is checked), units above 3 bits per symbol (squeezed in
+place), lanes that outgrow their slice (the unit is coded a second time), length quanta of two
+words, ragged last units, and tensors whose units do not fill the GPU evenly."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+from tests import nzabi as A
+
+pytestmark = pytest.mark.gpu
+
+
+def bits_of(kind, n, seed):
+    rng = np.random.default_rng(seed)
+    sign_mantissa = rng.integers(0, 256, n).astype(np.uint16)
+    if kind == "peaked":
+        exp = np.where(rng.random(n) < 0.9, 120, rng.integers(110, 125, n))
+    elif kind == "single":
+        exp = np.full(n, 121)
+    elif kind == "uniform10":                      # 3.3 bits per symbol
+        exp = rng.integers(115, 125, n)
+    elif kind == "uniform60":                      # 5.9 bits: every lane outgrows its slice
+        exp = rng.integers(80, 140, n)
+    else:                                          # one lane of 32 has the rare exponents
+        lane = (np.arange(n) // 8) % 32
+        exp = np.where(lane == 5, rng.integers(60, 180, n), np.where(rng.random(n) < 0.9, 120, 119))
+    exp = exp.astype(np.uint16)
+    return ((sign_mantissa & 0x80) << 8) | (exp << 7) | (sign_mantissa & 0x7F)
+
+
+@pytest.mark.parametrize("s", (7, 3, 1, 0))
+@pytest.mark.parametrize("kind", ("peaked", "single", "uniform10", "uniform60", "lane"))
+def test_encoder_branches(s, kind):
+    for S in (8, 64, 256, 776, 1024):
+        for n in (1, 32 * S, 32 * S * 5 + 3, 32 * S * 9 + 261):
+            bits = bits_of(kind, n, 7 * S + n % 11)
+            cont, frac, _ = A.compress(A.from_bits(bits), s, S)
+            c_ref, f_ref = O.compress_bf16(bits, s, S)
+            assert np.array_equal(cont.cpu().numpy(), c_ref), (s, kind, S, n)
+            assert np.array_equal(frac.cpu().numpy(), f_ref), (s, kind, S, n)
+
+
+def test_many_units_per_warp():
+    n = 32 * 8 * 148 * 48 * 3 + 1001
+    bits = bits_of("peaked", n, 3)
+    cont, frac, _ = A.compress(A.from_bits(bits), 7, 8)
+    c_ref, f_ref = O.compress_bf16(bits, 7, 8)
+    assert np.array_equal(cont.cpu().numpy(), c_ref) and np.array_equal(frac.cpu().numpy(), f_ref)
