@@ -415,6 +415,21 @@ __device__ __forceinline__ uint64_t frac_from_ring(uint32_t addr) {
 
 constexpr int kChains = NZ_DECODE_CHAINS;        // units a warp decodes side by side
 
+constexpr uint32_t kRingSlots = 4;               // blocks of fractions in flight per unit + 1
+// Shared-memory ring of a warp for the packed fractions, by precision.  One unit's
+// place holds, for precisions 7 and 3, one block (32 lanes x 8 or 4 bytes; four such
+// slots) and, for precisions 1 and 0, a group of four blocks (32 lanes x 8 or 4
+// bytes; two buffers).
+__host__ __device__ constexpr uint32_t ring_unit_bytes(int precision) {
+  return (precision == 7 || precision == 1) ? 256u : 128u;
+}
+__host__ __device__ constexpr uint32_t ring_warp_bytes(int precision) {
+  return ((precision == 7 || precision == 3) ? kRingSlots : 2u) * kChains *
+         ring_unit_bytes(precision);
+}
+// Precisions whose ring is filled block by block, per lane (the others: group by group).
+__host__ __device__ constexpr bool ring_by_block(int s) { return s == 7 || s == 3; }
+
 // What a warp knows about a unit it has planned.
 struct UnitPlan {
   uint32_t kind;       // 0 = nothing to do, 1 = raw, 2 = coded

@@ -189,19 +189,6 @@ __device__ __forceinline__ void emit_guarded(uint32_t sym, uint64_t e, int64_t d
 }
 
 constexpr int kFastRow = 7;                      // 128-byte table rows: one copy per bank
-constexpr uint32_t kRingSlots = 4;               // blocks of fractions in flight per unit + 1
-// Shared-memory ring of a warp for the packed fractions, by precision.  One unit's
-// place holds, for precisions 7 and 3, one block (32 lanes x 8 or 4 bytes; four such
-// slots) and, for precisions 1 and 0, a group of four blocks (32 lanes x 8 or 4
-// bytes; two buffers).
-__host__ __device__ constexpr uint32_t ring_unit_bytes(int precision) {
-  return (precision == 7 || precision == 1) ? 256u : 128u;
-}
-__host__ __device__ constexpr uint32_t ring_warp_bytes(int precision) {
-  return ((precision == 7 || precision == 3) ? kRingSlots : 2u) * kChains *
-         ring_unit_bytes(precision);
-}
-
 // Where the four words (8 bf16) that a lane produces per block and chain go.
 // StoreSink writes them to the output tensor.
 // ADV = elements between a lane's consecutive blocks: 256, or 64 in operand order (a
@@ -368,7 +355,6 @@ struct UpdateSinkT {
 // Start the copies of a group's first packed fractions into the warp's ring.  They depend on
 // nothing that is decoded, so the caller issues them before it waits for the coded units:
 // the two latencies overlap.  `ring` carries the lane's offset in a block (8 or 4 bytes).
-__host__ __device__ constexpr bool ring_by_block(int s) { return s == 7 || s == 3; }
 // s = 0 and 1: block counts that are a multiple of four go through the grouped ring
 __device__ __forceinline__ bool ring_by_group(int s, uint32_t n_blocks) {
   return (s == 0 || s == 1) && (n_blocks & 3) == 0;

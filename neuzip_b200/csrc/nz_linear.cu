@@ -62,6 +62,7 @@ struct LinearArgs {
   uint32_t slot_bytes;
   uint32_t lut_shift, lut_bytes;
   uint32_t stages;            // ring depth
+  uint32_t frac_ring;         // 1: the packed fractions go through shared memory
   uint32_t n_pad;             // MMA N: tokens of this launch, padded to a multiple of 16
   uint32_t n_tok;             // tokens of this launch that exist
   uint32_t tok0;              // first token of this launch
@@ -186,96 +187,128 @@ __device__ __forceinline__ void chain_symbols(LinChain &ch, const LutView &lv, u
 #pragma unroll
     for (int t = 0; t < 8; ++t) ent[t] = decode_step<kAnyRow>(ch.st, lv);
   } else {
-    const uint2 q = __ldg(reinterpret_cast<const uint2 *>(ch.raw));
+    // units start on any 16-bit word of the payload
+    const uint16_t *src = reinterpret_cast<const uint16_t *>(ch.raw);
     ch.raw += 256;
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
-      ent[t] = ((q.x >> (8 * t)) & 0xFFu) << kEntSymShift;
-      ent[t + 4] = ((q.y >> (8 * t)) & 0xFFu) << kEntSymShift;
+      const uint32_t pair = __ldg(src + t);
+      ent[2 * t] = (pair & 0xFFu) << kEntSymShift;
+      ent[2 * t + 1] = (pair >> 8) << kEntSymShift;
     }
   }
 }
 
+// The packed fractions of the two chains: through a ring in shared memory filled three blocks
+// ahead by asynchronous copies (as in decode_blocks_multi), or, where `ring` is 0 (precisions 1
+// and 0, or no room beside the operand tiles), loaded a block ahead into registers.
+template <int S>
+__device__ __forceinline__ void linear_ring_prologue(const LinChain (&ch)[2], uint32_t n_blocks,
+                                                     uint32_t ring) {
+  if (!ring_by_block(S) || !ring) return;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      if (ch[c].kind != kUnitSkip && (uint32_t)k < n_blocks)
+        frac_async<S>(ring + (k * 2 + c) * ring_unit_bytes(S), ch[c].frac + k * 32u * (S + 1));
+    frac_commit();
+  }
+}
+
+// One block per trip: the loop is fetched once per CTA and runs 16 to 48 times, so a longer
+// trip costs more in instruction fetches than it saves in loop overhead.
 template <int S, int ROW, bool BOTH_CODED>
 __device__ __forceinline__ bool linear_decode_loop(LinChain (&ch)[2], const LutView &lv, bool canon,
-                                                   uint32_t n_blocks, uint32_t stages,
+                                                   uint32_t n_blocks, uint32_t stages, uint32_t ring,
                                                    uint32_t tiles0, uint32_t bar_full0,
                                                    uint32_t bar_empty0, uint32_t lane,
                                                    const volatile uint32_t *abort_flag) {
   constexpr uint32_t kFracStride = 32u * (S + 1);
-  constexpr int kAhead = 4;
-  uint64_t fr[2][kAhead];
+  constexpr uint32_t kSlotBytes = 2 * ring_unit_bytes(S);
+  const bool by_ring = ring_by_block(S) && ring != 0;
+  uint64_t next[2] = {0, 0};
+  if (!by_ring) {
 #pragma unroll
-  for (int c = 0; c < 2; ++c)
-#pragma unroll
-    for (int k = 0; k < kAhead; ++k)
-      fr[c][k] = (ch[c].kind != kUnitSkip && (uint32_t)k < n_blocks)
-                     ? load_frac<S>(ch[c].frac + k * kFracStride) : 0;
-  uint32_t stage = 0, phase = 0;
+    for (int c = 0; c < 2; ++c)
+      if (ch[c].kind != kUnitSkip) next[c] = load_frac<S>(ch[c].frac);
+  }
+  uint32_t stage = 0, phase = 0, slot = 0;
 #pragma unroll 1
-  for (uint32_t b0 = 0; b0 < n_blocks; b0 += kAhead) {
+  for (uint32_t b = 0; b < n_blocks; ++b) {
+    uint64_t bits[2];
+    if (by_ring) {
+      const uint32_t ahead = (slot + 3 * kSlotBytes) & (4 * kSlotBytes - 1);
 #pragma unroll
-    for (int k = 0; k < kAhead; ++k) {
-      const uint32_t b = b0 + k;
-      if (b >= n_blocks) break;
-      uint64_t bits[2];
+      for (int c = 0; c < 2; ++c)
+        if ((BOTH_CODED || ch[c].kind != kUnitSkip) && b + 3 < n_blocks)
+          frac_async<S>(ring + ahead + c * ring_unit_bytes(S), ch[c].frac + 3 * kFracStride);
+      frac_commit();
+      frac_wait<3>();
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        bits[c] = fr[c][k];
-        if (ch[c].kind != kUnitSkip && b + kAhead < n_blocks)
-          fr[c][k] = load_frac<S>(ch[c].frac + (kAhead + k) * kFracStride);
-      }
-      uint32_t w[2][4];
-      if (BOTH_CODED) {
-        // the two chains' steps alternate: each hides the other's table and multiply latency
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          uint32_t e0[2], e1[2];
-#pragma unroll
-          for (int c = 0; c < 2; ++c) e0[c] = decode_step<ROW, usual_prob_bits(S)>(ch[c].st, lv);
-#pragma unroll
-          for (int c = 0; c < 2; ++c) e1[c] = decode_step<ROW, usual_prob_bits(S)>(ch[c].st, lv);
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            w[c][t] = merge_word<S, ROW>(e0[c], e1[c], bits[c], t);
-            if (ROW == 0 && canon) w[c][t] = canon_word(w[c][t]);
-          }
-        }
-      } else {
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          if (ch[c].kind == kUnitSkip) continue;
-          uint32_t ent[8];
-          chain_symbols(ch[c], lv, ent);
-#pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            w[c][t] = merge_word<S>(ent[2 * t], ent[2 * t + 1], bits[c], t);
-            if (canon) w[c][t] = canon_word(w[c][t]);
-          }
-        }
-      }
-      // the tensor cores must be done with the tile this step overwrites
-      if (b >= stages && !wait_phase_warp(bar_empty0 + 8 * stage, phase ^ 1, abort_flag)) return false;
-      const uint32_t tile = tiles0 + stage * kTileBytes;
+      for (int c = 0; c < 2; ++c) bits[c] = frac_from_ring<S>(ring + slot + c * ring_unit_bytes(S));
+      slot = (slot + kSlotBytes) & (4 * kSlotBytes - 1);
+    } else {
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
-        if (!BOTH_CODED && ch[c].kind == kUnitSkip) continue;
-        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(tile + ch[c].dst),
-                     "r"(w[c][0]), "r"(w[c][1]), "r"(w[c][2]), "r"(w[c][3])
-                     : "memory");
-      }
-      // make this lane's stores visible to the tensor cores' (asynchronous proxy) reads,
-      // then one arrival per warp
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_full0 + 8 * stage);
-      if (++stage == stages) {
-        stage = 0;
-        phase ^= 1;
+        bits[c] = next[c];
+        if ((BOTH_CODED || ch[c].kind != kUnitSkip) && b + 1 < n_blocks)
+          next[c] = load_frac<S>(ch[c].frac + kFracStride);
       }
     }
 #pragma unroll
-    for (int c = 0; c < 2; ++c) ch[c].frac += kAhead * kFracStride;
+    for (int c = 0; c < 2; ++c) ch[c].frac += kFracStride;
+    uint32_t w[2][4];
+    if (BOTH_CODED) {
+      // the two chains' steps alternate: each hides the other's table and multiply latency
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        uint32_t e0[2], e1[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) e0[c] = decode_step<ROW, usual_prob_bits(S)>(ch[c].st, lv);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) e1[c] = decode_step<ROW, usual_prob_bits(S)>(ch[c].st, lv);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          w[c][t] = merge_word<S, ROW>(e0[c], e1[c], bits[c], t);
+          if (ROW == 0 && canon) w[c][t] = canon_word(w[c][t]);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        if (ch[c].kind == kUnitSkip) continue;
+        uint32_t ent[8];
+        chain_symbols(ch[c], lv, ent);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          w[c][t] = merge_word<S>(ent[2 * t], ent[2 * t + 1], bits[c], t);
+          if (canon) w[c][t] = canon_word(w[c][t]);
+        }
+      }
+    }
+    // the tensor cores must be done with the tile this step overwrites
+    if (b >= stages && !wait_phase_warp(bar_empty0 + 8 * stage, phase ^ 1, abort_flag)) {
+      frac_wait<0>();
+      return false;
+    }
+    const uint32_t tile = tiles0 + stage * kTileBytes;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      if (!BOTH_CODED && ch[c].kind == kUnitSkip) continue;
+      asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(tile + ch[c].dst),
+                   "r"(w[c][0]), "r"(w[c][1]), "r"(w[c][2]), "r"(w[c][3])
+                   : "memory");
+    }
+    // make this lane's stores visible to the tensor cores' (asynchronous proxy) reads,
+    // then one arrival per warp
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar_full0 + 8 * stage);
+    if (++stage == stages) {
+      stage = 0;
+      phase ^= 1;
+    }
   }
   return true;
 }
@@ -284,6 +317,7 @@ __device__ __forceinline__ bool linear_decode_loop(LinChain (&ch)[2], const LutV
 //   [0, lut_bytes)                      decode table
 //   [lut_bytes, +1024)                  mbarriers, scan scratch, flags
 //   [.., + 32 * slot_bytes + guard)     staged units
+//   [.., + 16 * ring_warp_bytes)        rings for the packed fractions (when there is room)
 //   (1024-aligned) stages x 16 KB       weight tiles
 //   (1024-aligned) stages x n_pad*128   x slabs
 constexpr uint32_t kBarWarp = 0;         // 16 x 8 bytes: per-warp staging barriers
@@ -343,7 +377,9 @@ linear_kernel(const LinearArgs p, const __grid_constant__ CUtensorMap x_map) {
   volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(misc + kTmemSlot);
   const uint32_t guard = ((p.S + 8) * 2 + 127) & ~127u;
   const uint32_t slots_a = misc_a + 1024;
-  const uint32_t tiles_a = (slots_a + 2 * kLinDecWarps * p.slot_bytes + guard + 1023u) & ~1023u;
+  const uint32_t rings_a = slots_a + 2 * kLinDecWarps * p.slot_bytes + guard;
+  const uint32_t tiles_a =
+      (rings_a + (p.frac_ring ? kLinDecWarps * ring_warp_bytes(S) : 0u) + 1023u) & ~1023u;
   const uint32_t xslab_bytes = p.n_pad * 128u;
   const uint32_t xs_a = tiles_a + p.stages * kTileBytes;     // 16 KB tiles keep this 1024-aligned
   const uint32_t n_blocks = p.S / 8;
@@ -379,6 +415,11 @@ linear_kernel(const LinearArgs p, const __grid_constant__ CUtensorMap x_map) {
   }
   __syncwarp();
 
+  // The launch may overlap the tail of the kernel before it (programmatic stream
+  // serialisation): barriers, flags and tensor memory are set up by now, global memory is not
+  // touched before that kernel has completed.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+
   // ---- plan and stage this warp's two units, build the decode table meanwhile
   const Header *h = reinterpret_cast<const Header *>(a.container);
   const uint32_t bar_w = misc_a + kBarWarp + 8 * (is_dec ? warp : 0);
@@ -409,8 +450,8 @@ linear_kernel(const LinearArgs p, const __grid_constant__ CUtensorMap x_map) {
   LutView lv;
   uint32_t row_shift = 0;
   const bool canon = a.canon && (cum_sh[256] != cum_sh[255]);
-  // row sizes with a loop for narrow entries (see decode_kernel)
-  const uint32_t narrow_rows = canon ? 0u : (1u << 7) | (S != 7 ? 1u << 6 : 0u);
+  // row sizes with a loop for narrow entries: 32 or 16 copies of the usual table
+  const uint32_t narrow_rows = canon ? 0u : (1u << 7) | (1u << 6);
   if (ok) table_fill(a.lut_shift, a.S, pb, smem, cum_sh, narrow_rows, usual_prob_bits(S), flag_sh, warp,
                      lane, kLinWarps, lv, row_shift);
   else if (threadIdx.x == 0 && blockIdx.x == 0) raise(a.status, bad);
@@ -418,34 +459,45 @@ linear_kernel(const LinearArgs p, const __grid_constant__ CUtensorMap x_map) {
 
   if (is_dec) {
     // ---------------------------------------------------------------- decoder warps
+    LinChain ch[2];
+    const uint64_t U = 32ull * a.S;
+    const uint32_t lenq = len_quantum(a.S);
+    const uint32_t ring =
+        p.frac_ring ? rings_a + warp * ring_warp_bytes(S) + lane * (S == 7 ? 8u : 4u) : 0u;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      ch[c].kind = ok ? pl[c].kind : kUnitSkip;
+      ch[c].raw = a.container + a.pay_off + pl[c].byte0() + lane * 8;
+      ch[c].st.x = kStateLow;
+      ch[c].st.p = slot0;
+      ch[c].st.w = 0;
+      const uint64_t e = (uint64_t)unit[c] * U + lane * 8;        // stream order
+      ch[c].frac = a.frac + e * (S + 1) / 8;
+      const uint32_t r = 4 * (2 * warp + c) + (lane >> 3);        // row inside the tile
+      ch[c].dst = r * 128u + (((lane & 7u) ^ (r & 7u)) << 4);
+    }
+    // the first fractions are on their way while the units arrive
+    linear_ring_prologue<S>(ch, n_blocks, ring);
     if (staged && !__all_sync(0xFFFFFFFFu, wait_staged(bar_w, 0))) {
       if (lane == 0) raise(a.status, NZ_STATUS_TIMEOUT);
       *abort_flag = 1;
       ok = false;
+      frac_wait<0>();
     }
     if (ok) {
-      LinChain ch[2];
-      const uint64_t U = 32ull * a.S;
-      const uint32_t lenq = len_quantum(a.S);
+      LaneState st[2];
+      if (ch[0].kind == kUnitCoded && ch[1].kind == kUnitCoded &&
+          open_pair(pl, slot0, a.slot_bytes, lenq, lane, st)) {
+        ch[0].st = st[0];
+        ch[1].st = st[1];
+      } else {
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        ch[c].kind = pl[c].kind;
-        ch[c].raw = nullptr;
-        ch[c].st.x = kStateLow;
-        ch[c].st.p = slot0;
-        ch[c].st.w = 0;
-        if (pl[c].kind == kUnitCoded) {
-          if (!open_unit(pl[c], slot0 + c * a.slot_bytes, lenq, lane, ch[c].st)) {
+        for (int c = 0; c < 2; ++c)
+          if (ch[c].kind == kUnitCoded &&
+              !open_unit(pl[c], slot0 + c * a.slot_bytes, lenq, lane, ch[c].st)) {
             if (lane == 0) raise(a.status, NZ_STATUS_BAD_LANES);
             ch[c].kind = kUnitSkip;
           }
-        } else if (pl[c].kind == kUnitRaw) {
-          ch[c].raw = a.container + a.pay_off + pl[c].byte0() + lane * 8;
-        }
-        const uint64_t e = (uint64_t)unit[c] * U + lane * 8;        // stream order
-        ch[c].frac = a.frac + e * (S + 1) / 8;
-        const uint32_t r = 4 * (2 * warp + c) + (lane >> 3);        // row inside the tile
-        ch[c].dst = r * 128u + (((lane & 7u) ^ (r & 7u)) << 4);
       }
       // Units that cannot be decoded leave their rows of the tile as they are: a row of
       // the operand only ever reaches the same row of the result, which is not stored
@@ -454,13 +506,13 @@ linear_kernel(const LinearArgs p, const __grid_constant__ CUtensorMap x_map) {
       const bool both = ch[0].kind == kUnitCoded && ch[1].kind == kUnitCoded;
       bool fine;
 #define NZ_LIN_LOOP(ROW, BOTH)                                                                 \
-  linear_decode_loop<S, ROW, BOTH>(ch, lv, canon, n_blocks, p.stages, tiles_a, bar_full0,      \
-                                   bar_empty0, lane, abort_flag)
+  linear_decode_loop<S, ROW, BOTH>(ch, lv, canon, n_blocks, p.stages, ring, tiles_a,           \
+                                   bar_full0, bar_empty0, lane, abort_flag)
       if (!both)
         fine = NZ_LIN_LOOP(0, false);
       else if (lv.narrow && row_shift == 7)
         fine = NZ_LIN_LOOP(7, true);
-      else if (S != 7 && lv.narrow)
+      else if (lv.narrow)
         fine = NZ_LIN_LOOP(6, true);
       else
         fine = NZ_LIN_LOOP(0, true);
@@ -643,7 +695,8 @@ __global__ void linear_finish_kernel(const float *__restrict__ partial, uint32_t
                                      const uint16_t *__restrict__ bias, uint16_t *__restrict__ y) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   // launched with programmatic stream serialisation: wait for the kernel that wrote the
-  // partial sums (a no-op for an ordinary launch)
+  // partial sums (a no-op for an ordinary launch); the next launch may be set up meanwhile
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (i >= plane) return;
   float sum = 0.f;
@@ -719,10 +772,11 @@ static uint32_t operand_segments(uint64_t cols, uint32_t S) {
 }
 
 struct LinearGeometry {
-  uint32_t slot_bytes, lut_shift, stages, smem_bytes;
+  uint32_t slot_bytes, lut_shift, stages, frac_ring, smem_bytes;
 };
 
-static bool linear_geometry(uint32_t S, uint32_t max_unit_words, uint32_t n_pad, LinearGeometry &g) {
+static bool linear_geometry(uint32_t S, uint32_t max_unit_words, uint32_t n_pad, int precision,
+                            LinearGeometry &g) {
   const uint64_t U = 32ull * S;
   uint64_t unit_bytes = max_unit_words ? (uint64_t)max_unit_words * 2 : U;
   if (unit_bytes > U) unit_bytes = U;
@@ -732,8 +786,7 @@ static bool linear_geometry(uint32_t S, uint32_t max_unit_words, uint32_t n_pad,
   const uint32_t fixed = 1024 /* alignment slack */ + 1024 /* misc */ +
                          2 * kLinDecWarps * g.slot_bytes + guard + 1024 /* tile alignment */;
   const uint32_t per_stage = kTileBytes + n_pad * 128u;
-  // Ring depth first (decoder warps that run ahead of the slowest one need somewhere to
-  // write), then table copies (fewer shared-memory bank conflicts per lookup).
+  const uint32_t rings = ring_by_block(precision) ? kLinDecWarps * ring_warp_bytes(precision) : 0;
   const char *force = getenv("NZ_LINEAR_GEOMETRY");      // "<lut_shift>,<stages>": tuning aid
   if (force) {
     unsigned sh = 0, st = 0;
@@ -742,17 +795,25 @@ static bool linear_geometry(uint32_t S, uint32_t max_unit_words, uint32_t n_pad,
       if (need <= kMaxDynamicSmem) {
         g.lut_shift = sh;
         g.stages = st;
-        g.smem_bytes = (uint32_t)need;
+        g.frac_ring = rings && need + rings <= kMaxDynamicSmem;
+        g.smem_bytes = (uint32_t)need + (g.frac_ring ? rings : 0);
         return true;
       }
     }
   }
-  static const uint32_t order[][2] = {{4, 3}, {3, 3}, {4, 2}, {3, 2}, {2, 3}, {2, 2}};
+  // {table copies, ring depth, fraction rings}: the table's 32 (16) copies of the usual
+  // resolution first, then the fraction rings, then a third operand stage (decoder warps that
+  // run ahead of the slowest one need somewhere to write)
+  static const uint32_t order[][3] = {{4, 3, 1}, {4, 2, 1}, {4, 3, 0}, {4, 2, 0}, {3, 3, 1}, {3, 2, 1},
+                                      {3, 3, 0}, {3, 2, 0}, {2, 3, 0}, {2, 2, 0}};
   for (const auto &o : order) {
-    const uint64_t need = (uint64_t)fixed + (4096u << o[0]) + (uint64_t)o[1] * per_stage;
+    if (o[2] && !rings) continue;
+    const uint64_t need =
+        (uint64_t)fixed + (4096u << o[0]) + (uint64_t)o[1] * per_stage + (o[2] ? rings : 0);
     if (need <= kMaxDynamicSmem) {
       g.lut_shift = o[0];
       g.stages = o[1];
+      g.frac_ring = o[2];
       g.smem_bytes = (uint32_t)need;
       return true;
     }
@@ -884,7 +945,7 @@ static int linear_impl(const void *container, uint64_t container_bytes, const vo
       (uint32_t)(m_tokens < kMaxTokensPerLaunch ? m_tokens : kMaxTokensPerLaunch);
   const uint32_t n_pad = (per_launch + 15u) & ~15u;
   LinearGeometry g;
-  if (!linear_geometry(lane_symbols, max_unit_words, n_pad, g)) {
+  if (!linear_geometry(lane_symbols, max_unit_words, n_pad, precision, g)) {
     set_error("nz_linear_bf16: units of lane_symbols %u do not fit in shared memory next to the "
               "operand tiles", lane_symbols);
     return NZ_E_CAPACITY;
@@ -921,6 +982,7 @@ static int linear_impl(const void *container, uint64_t container_bytes, const vo
   p.lut_shift = g.lut_shift;
   p.lut_bytes = 4096u << g.lut_shift;
   p.stages = g.stages;
+  p.frac_ring = g.frac_ring;
   p.n_pad = n_pad;
   p.m_total = (uint32_t)m_tokens;
   p.tmem_cols = 32;
@@ -974,6 +1036,11 @@ static int linear_impl(const void *container, uint64_t container_bytes, const vo
     cfg.blockDim = dim3(kLinThreads);
     cfg.dynamicSmemBytes = g.smem_bytes;
     cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
     NZ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p, x_map));
   }
   if (peers) {

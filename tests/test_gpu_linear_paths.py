@@ -1,0 +1,72 @@
+"""Branches of the fused linear: raw units between coded ones (their bytes start on any 16-bit
+word), shapes with and without room for the fraction rings beside the operand tiles, and calls
+back to back on one workspace (the launches overlap)."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+from tests import nzabi as A
+
+pytestmark = pytest.mark.gpu
+
+
+def reference(w, x):
+    return (x.double() @ w.double().t()).cpu()
+
+
+def check(y, ref):
+    # fp32 sums rounded once to bf16: half a unit in the last place (2^-9 of the value) and the
+    # fp32 accumulation, bounded by the largest result
+    err = (y.double().cpu() - ref).abs()
+    assert bool((err <= 2.0 ** -8 * ref.abs() + 2.0 ** -14 * ref.abs().max()).all())
+
+
+@pytest.mark.parametrize("s", (7, 3, 0))
+def test_raw_units_between_coded_ones(s):
+    rows, cols, S = 132, 2048, 128
+    g = torch.Generator().manual_seed(s)
+    w = (torch.randn(rows, cols, generator=g) * 0.02).to(torch.bfloat16)
+    bits = A.to_bits(w).reshape(rows, cols).copy()
+    rng = np.random.default_rng(3)
+    for row in (0, 20, 64, 100):                     # row groups whose exponents do not compress
+        bits[row:row + 4, :1024] = ((rng.integers(1, 250, (4, 1024)) << 7) | (bits[row:row + 4, :1024] & 0x807F))
+    bits[np.isin(bits >> 7 & 0xFF, (255,))] = 0
+    # keep the products finite: large exponents only against zero inputs
+    x = torch.randn(16, cols, generator=g).to(torch.bfloat16)
+    x[:, :1024] = 0
+    x[:, 7] = 2.0 ** -100
+    wt = A.from_bits(bits.reshape(-1))
+    cont, frac, mw = A.compress_operand(wt, rows, cols, s, S)
+    offs = np.frombuffer(cont.cpu().numpy().tobytes(), dtype=np.uint32, count=rows // 4 * 2 + 1, offset=576)
+    raw = offs[:-1] >> 31 == 1
+    assert raw.any() and not raw.all() and (offs[:-1][raw] & 1).any()     # some at odd words
+    stored = A.decompress_operand(cont, frac, rows, cols, s, S)[0].view(rows, cols)
+    y, status = A.linear(cont, frac, rows, cols, s, S, x.cuda(), max_words=mw)
+    assert status == 0
+    keep = torch.ones(rows, dtype=torch.bool)
+    for row in (0, 20, 64, 100):
+        keep[row:row + 4] = False
+    check(y.cpu()[:, keep], reference(stored.cpu(), x)[:, keep])
+    check(y.cpu()[:, ~keep].clamp(-1e30, 1e30), reference(stored.cpu(), x)[:, ~keep].clamp(-1e30, 1e30))
+
+
+@pytest.mark.parametrize("m", (1, 17, 256))
+@pytest.mark.parametrize("cols,S", ((2048, 128), (11008, 344), (4096, 256)))
+def test_with_and_without_room_for_the_rings(cols, S, m):
+    rows = 260
+    g = torch.Generator().manual_seed(cols + m)
+    w = (torch.randn(rows, cols, generator=g) * 0.02).to(torch.bfloat16).cuda()
+    x = torch.randn(m, cols, generator=g).to(torch.bfloat16).cuda()
+    for s in (7, 3):
+        cont, frac, mw = A.compress_operand(w, rows, cols, s, S)
+        stored = A.decompress_operand(cont, frac, rows, cols, s, S)[0].view(rows, cols)
+        if S == 344 and m == 256:
+            continue                              # units too long beside this many input rows
+        ys = []
+        for _ in range(3):
+            y, status = A.linear(cont, frac, rows, cols, s, S, x, max_words=mw)
+            assert status == 0
+            ys.append(y)
+        check(ys[0].cpu(), reference(stored.cpu(), x.cpu()))
+        assert all(torch.equal(ys[0], y) for y in ys)
