@@ -60,6 +60,10 @@ static inline uint64_t work_units(const HostItem &it) {
 // (17 cycles per warp-symbol) or its shared-memory pipe (2.7 wavefronts and one table
 // lookup, in which 32 / copies lanes share a bank) need.  Without a loop for narrow rows
 // (`narrow` false) the chains of a warp hardly overlap.
+//
+// A tensor with so few units that every one can have a warp of its own (20 per SM) is decoded
+// with one chain per warp instead of two: a step then takes the latency of one chain (73
+// cycles on a B200, 107 with two chains in a lone warp), on twice as many warps.
 static uint32_t step_cycles(uint32_t w, uint32_t copies, bool narrow) {
   const uint32_t issue = (narrow ? 34 : 40) * ((w + 3) / 4);
   const uint32_t wavefronts10 = 27 + (copies >= 32 ? 10 : copies >= 16 ? 20 : copies >= 8 ? 35 : 50);
@@ -82,7 +86,7 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
   const uint32_t sm_smem = 227u * 1024u;
   const uint32_t max_warps = items[0].gx ? (uint32_t)kDotMaxWarps
                              : items[0].grad ? (uint32_t)kUpdateMaxWarps : (uint32_t)NZ_DECODE_MAX_WARPS;
-  uint64_t total_work = 0, total_groups = 0;
+  uint64_t total_work = 0, total_units = 0;
   uint32_t groups[kMaxBatch], guard[kMaxBatch], per_warp[kMaxBatch];
   for (uint32_t t = 0; t < count; ++t) {
     const uint64_t U = 32ull * items[t].S;
@@ -97,18 +101,18 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
       return NZ_E_ARG;
     }
     groups[t] = (uint32_t)((work_units(items[t]) + kChains - 1) / kChains);
-    total_groups += groups[t];
+    total_units += work_units(items[t]);
     total_work += (uint64_t)groups[t] * items[t].S;
   }
   // CTAs per tensor: one per SM (fewer when there is not enough work to give every SM a
-  // group of units), in proportion to the symbols, at least one
+  // unit), in proportion to the symbols, at least one
   uint32_t n_ctas = (uint32_t)sm_count();
-  if (total_groups < n_ctas) n_ctas = (uint32_t)total_groups;
+  if (total_units < n_ctas) n_ctas = (uint32_t)total_units;
   if (n_ctas < count) n_ctas = count;
   uint32_t share[kMaxBatch], used = 0;
   for (uint32_t t = 0; t < count; ++t) {
     uint64_t c = total_work ? (uint64_t)groups[t] * items[t].S * n_ctas / total_work : 1;
-    if (c > groups[t]) c = groups[t];
+    if (c > work_units(items[t])) c = work_units(items[t]);
     if (c < 1) c = 1;
     share[t] = (uint32_t)c;
     used += share[t];
@@ -147,7 +151,7 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
         for (uint32_t t = 1; t < count; ++t)
           if (cost(t, now[t]) > cost(hi, now[hi])) hi = t;
         if (sum < n_ctas) {
-          if (now[hi] >= groups[hi]) break;
+          if (now[hi] >= work_units(items[hi])) break;
           ++now[hi];
           ++sum;
           continue;
@@ -162,7 +166,7 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
           --sum;
           continue;
         }
-        if (now[hi] >= groups[hi] || cost(lo, now[lo] - 1) >= cost(hi, now[hi])) break;
+        if (now[hi] >= work_units(items[hi]) || cost(lo, now[lo] - 1) >= cost(hi, now[hi])) break;
         --now[lo];
         ++now[hi];
       }
@@ -187,18 +191,30 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
     BatchItem &it = b.item[t];
     // no more warps than make the rounds even, and a second staging buffer per warp where
     // there is more than one round and room for it
-    const uint32_t g = (groups[t] + ctas[t] - 1) / ctas[t];
-    const uint32_t rounds = (g + it.warps - 1) / it.warps;
-    it.warps = (g + rounds - 1) / rounds;
-    const uint32_t fixed = b.lut_bytes + guard[t] + it.warps * ring_bytes;
-    const uint32_t slots = it.warps * kChains * it.slot_bytes;
-    it.bufs = rounds > 1 && fixed + 2 * slots <= sm_smem ? 2u : 1u;
-    it.ring_offset = b.lut_bytes + guard[t] + it.bufs * slots;
+    const uint64_t units = work_units(items[t]);
+    const uint32_t own = (uint32_t)((units + ctas[t] - 1) / ctas[t]);     // units per CTA
+    const uint32_t fixed0 = b.lut_bytes + guard[t];
+    if (!items[0].gx && !items[0].grad && own <= max_warps &&
+        fixed0 + own * (it.slot_bytes + ring_bytes) <= sm_smem) {
+      it.chains = 1;
+      it.warps = own;
+      it.bufs = 1;
+      it.groups_each = (uint32_t)units / (ctas[t] * it.warps);
+      it.groups_more = (uint32_t)units % (ctas[t] * it.warps);
+    } else {
+      const uint32_t g = (groups[t] + ctas[t] - 1) / ctas[t];
+      const uint32_t rounds = (g + it.warps - 1) / it.warps;
+      it.chains = kChains;
+      it.warps = (g + rounds - 1) / rounds;
+      it.bufs = rounds > 1 && fixed0 + it.warps * (ring_bytes + 2 * kChains * it.slot_bytes) <= sm_smem
+                    ? 2u : 1u;
+      it.groups_each = groups[t] / (ctas[t] * it.warps);
+      it.groups_more = groups[t] % (ctas[t] * it.warps);
+    }
+    it.ring_offset = fixed0 + it.bufs * it.warps * it.chains * it.slot_bytes;
     const uint32_t need = it.ring_offset + it.warps * ring_bytes;
     if (need > smem_bytes) smem_bytes = need;
     if (it.warps > warps) warps = it.warps;
-    it.groups_each = groups[t] / (ctas[t] * it.warps);
-    it.groups_more = groups[t] % (ctas[t] * it.warps);
     it.cta_begin = begin;
     begin += ctas[t];
   }

@@ -66,8 +66,9 @@ struct BatchItem {
   uint32_t tile_cols;     // operand order: row length (0 = stream order)
   uint32_t segs;          //   units per row group
   uint32_t S;             // lane symbols of this tensor
-  uint32_t groups_each;   // groups of kChains units per warp (one more for the first groups_more)
+  uint32_t groups_each;   // groups of `chains` units per warp (one more for the first groups_more)
   uint32_t groups_more;
+  uint32_t chains;        // units a warp decodes side by side: 2, or 1 when there are few
   uint32_t warps;         // warps of a CTA that decode (the others leave once the table is built)
   uint32_t bufs;          // staging buffers per warp, 1 or 2
   uint32_t slot_bytes;    // one unit's place in a buffer
@@ -359,7 +360,7 @@ struct UpdateSinkT {
 __device__ __forceinline__ bool ring_by_group(int s, uint32_t n_blocks) {
   return (s == 0 || s == 1) && (n_blocks & 3) == 0;
 }
-template <int S>
+template <int S, int C>
 __device__ __forceinline__ void group_async(uint32_t ring, const uint8_t *(&frac)[kChains],
                                             uint32_t g) {
   // four blocks of a unit are 128 (s=0) or 256 (s=1) contiguous bytes, copied by the whole
@@ -370,7 +371,7 @@ __device__ __forceinline__ void group_async(uint32_t ring, const uint8_t *(&frac
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t dst = ring - lane * 4 + (g & 1) * (kChains * kRingUnitBytes) + lane * kLaneBytes;
 #pragma unroll
-  for (int c = 0; c < kChains; ++c) {
+  for (int c = 0; c < C; ++c) {
     const uint8_t *src = frac[c] - lane * (S + 1) + (uint64_t)g * kGroupBytes + lane * kLaneBytes;
     if (S == 1)
       asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + c * kRingUnitBytes),
@@ -383,7 +384,7 @@ __device__ __forceinline__ void group_async(uint32_t ring, const uint8_t *(&frac
   }
   frac_commit();
 }
-template <int S>
+template <int S, int C>
 __device__ __forceinline__ void ring_prologue(uint32_t ring, const uint8_t *(&frac)[kChains],
                                               uint32_t n_blocks) {
   if (ring_by_block(S)) {
@@ -391,18 +392,18 @@ __device__ __forceinline__ void ring_prologue(uint32_t ring, const uint8_t *(&fr
     for (int k = 0; k < 3; ++k) {
       if ((uint32_t)k < n_blocks) {
 #pragma unroll
-        for (int c = 0; c < kChains; ++c)
+        for (int c = 0; c < C; ++c)
           frac_async<S>(ring + k * (kChains * ring_unit_bytes(S)) + c * ring_unit_bytes(S),
                         frac[c] + k * 32u * (S + 1));
       }
       frac_commit();
     }
   } else if (ring_by_group(S, n_blocks)) {
-    group_async<S>(ring, frac, 0);
+    group_async<S, C>(ring, frac, 0);
   }
 }
 
-// kChains units interleaved in one lane: the rANS chains are independent, so
+// C units (1 or 2) interleaved in one lane: the rANS chains are independent, so
 // each hides the shared-memory and multiply latency of the others.  For
 // precisions 3 and 7 the packed fractions travel through a small ring in shared
 // memory, fetched three blocks ahead with per-lane asynchronous copies; the
@@ -410,7 +411,7 @@ __device__ __forceinline__ void ring_prologue(uint32_t ring, const uint8_t *(&fr
 // are fetched four blocks at a time by the whole warp.  The caller has started the
 // first copies (ring_prologue); returns true when the next group's first copies are under
 // way in their place.
-template <int S, bool MERGE, int ROW, typename Sink>
+template <int S, bool MERGE, int ROW, int C, typename Sink>
 __device__ __forceinline__ bool decode_blocks_multi(LaneState (&st)[kChains], const LutView &lut,
                                                     uint32_t n_blocks, bool canon,
                                                     const uint8_t *(&frac)[kChains],
@@ -430,9 +431,9 @@ __device__ __forceinline__ bool decode_blocks_multi(LaneState (&st)[kChains], co
 #pragma unroll
       for (int t = 0; t < 8; ++t)
 #pragma unroll
-        for (int c = 0; c < kChains; ++c) e[c][t] = decode_step<ROW, usual_prob_bits(S)>(st[c], lut);
+        for (int c = 0; c < C; ++c) e[c][t] = decode_step<ROW, usual_prob_bits(S)>(st[c], lut);
 #pragma unroll
-      for (int c = 0; c < kChains; ++c) {
+      for (int c = 0; c < C; ++c) {
         store_exp_block<ROW>(e[c], exp[c]);
         exp[c] += 256;
       }
@@ -443,30 +444,30 @@ __device__ __forceinline__ bool decode_blocks_multi(LaneState (&st)[kChains], co
   // then their output words (the table entries do not stay live for the whole block).
   auto decode_block = [&](const uint64_t (&bits)[kChains], int k) {
 #pragma unroll
-    for (int c = 0; c < kChains; ++c) sink.begin(c);
+    for (int c = 0; c < C; ++c) sink.begin(c);
     uint32_t w[kChains][4];
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       uint32_t e0[kChains], e1[kChains];
 #pragma unroll
-      for (int c = 0; c < kChains; ++c) e0[c] = decode_step<ROW, usual_prob_bits(S)>(st[c], lut);
+      for (int c = 0; c < C; ++c) e0[c] = decode_step<ROW, usual_prob_bits(S)>(st[c], lut);
 #pragma unroll
-      for (int c = 0; c < kChains; ++c) e1[c] = decode_step<ROW, usual_prob_bits(S)>(st[c], lut);
+      for (int c = 0; c < C; ++c) e1[c] = decode_step<ROW, usual_prob_bits(S)>(st[c], lut);
 #pragma unroll
-      for (int c = 0; c < kChains; ++c) {
+      for (int c = 0; c < C; ++c) {
         w[c][t] = merge_word<S, ROW>(e0[c], e1[c], bits[c], t);
         if (ROW == 0 && canon) w[c][t] = canon_word(w[c][t]);
       }
     }
 #pragma unroll
-    for (int c = 0; c < kChains; ++c) sink.put(c, k, w[c]);
+    for (int c = 0; c < C; ++c) sink.put(c, k, w[c]);
   };
   if (ring_by_block(S)) {
     auto ring_read = [&](uint32_t at, uint64_t (&bits)[kChains]) {
       frac_commit();
       frac_wait<3>();
 #pragma unroll
-      for (int c = 0; c < kChains; ++c)
+      for (int c = 0; c < C; ++c)
         bits[c] = frac_from_ring<S>(ring + at + c * kRingUnitBytes);
     };
     // Block b starts the copy of block b + 3 into the ring slot that block b - 1 has left
@@ -477,7 +478,7 @@ __device__ __forceinline__ bool decode_blocks_multi(LaneState (&st)[kChains], co
     uint32_t b = 0;
     const uint8_t *fetch[kChains];
 #pragma unroll
-    for (int c = 0; c < kChains; ++c) fetch[c] = frac[c] + 3 * kFracStride;
+    for (int c = 0; c < C; ++c) fetch[c] = frac[c] + 3 * kFracStride;
     if (kTrip > 1) {
       const uint32_t fetch_end = carry ? ~0u : n_blocks;
       uint32_t half = 0;                       // byte offset of the trip's two ring slots
@@ -486,26 +487,26 @@ __device__ __forceinline__ bool decode_blocks_multi(LaneState (&st)[kChains], co
         uint64_t bits[kChains];
         if (b + 3 < fetch_end) {
 #pragma unroll
-          for (int c = 0; c < kChains; ++c)
+          for (int c = 0; c < C; ++c)
             frac_async<S>(ring + (half ^ (2 * kRingSlotBytes)) + kRingSlotBytes + c * kRingUnitBytes,
                           fetch[c]);
         }
         ring_read(half, bits);
         decode_block(bits, 0);
 #pragma unroll
-        for (int c = 0; c < kChains; ++c) {
+        for (int c = 0; c < C; ++c) {
           fetch[c] += kFracStride;
           if (carry && b + 4 == n_blocks) fetch[c] = next_frac[c];
         }
         if (b + 4 < fetch_end) {
 #pragma unroll
-          for (int c = 0; c < kChains; ++c)
+          for (int c = 0; c < C; ++c)
             frac_async<S>(ring + half + c * kRingUnitBytes, fetch[c]);
         }
         ring_read(half + kRingSlotBytes, bits);
         decode_block(bits, 1);
 #pragma unroll
-        for (int c = 0; c < kChains; ++c) fetch[c] += kFracStride;
+        for (int c = 0; c < C; ++c) fetch[c] += kFracStride;
         half ^= 2 * kRingSlotBytes;
         sink.advance(kTrip);
       }
@@ -514,7 +515,7 @@ __device__ __forceinline__ bool decode_blocks_multi(LaneState (&st)[kChains], co
     for (; b < n_blocks; ++b) {
       if (b + 3 < n_blocks) {
 #pragma unroll
-        for (int c = 0; c < kChains; ++c)
+        for (int c = 0; c < C; ++c)
           frac_async<S>(ring + ((b + 3) % kRingSlots) * kRingSlotBytes + c * kRingUnitBytes,
                         fetch[c]);
       }
@@ -522,7 +523,7 @@ __device__ __forceinline__ bool decode_blocks_multi(LaneState (&st)[kChains], co
       ring_read((b % kRingSlots) * kRingSlotBytes, bits);
       decode_block(bits, 0);
 #pragma unroll
-      for (int c = 0; c < kChains; ++c) fetch[c] += kFracStride;
+      for (int c = 0; c < C; ++c) fetch[c] += kFracStride;
       sink.advance(1);
     }
     return carry;
@@ -538,7 +539,7 @@ __device__ __forceinline__ bool decode_blocks_multi(LaneState (&st)[kChains], co
     for (uint32_t g = 0; g < n_groups; ++g) {
       __syncwarp();                       // everyone is done with the buffer about to be refilled
       if (g + 1 < n_groups) {
-        group_async<S>(ring, frac, g + 1);
+        group_async<S, C>(ring, frac, g + 1);
         frac_wait<1>();
       } else {
         frac_wait<0>();
@@ -548,7 +549,7 @@ __device__ __forceinline__ bool decode_blocks_multi(LaneState (&st)[kChains], co
       auto group_block = [&](int at, int k) {
         uint64_t bits[kChains];
 #pragma unroll
-        for (int c = 0; c < kChains; ++c)
+        for (int c = 0; c < C; ++c)
           bits[c] = (S == 1) ? lds_u16(src + c * kRingUnitBytes + at * 64)
                              : lds_u8(src + c * kRingUnitBytes + at * 32);
         decode_block(bits, k);
@@ -564,12 +565,12 @@ __device__ __forceinline__ bool decode_blocks_multi(LaneState (&st)[kChains], co
   }
   uint64_t next[kChains];
 #pragma unroll
-  for (int c = 0; c < kChains; ++c) next[c] = load_frac<S>(frac[c]);
+  for (int c = 0; c < C; ++c) next[c] = load_frac<S>(frac[c]);
 #pragma unroll 1
   for (; b < n_blocks; ++b) {
     uint64_t bits[kChains];
 #pragma unroll
-    for (int c = 0; c < kChains; ++c) {
+    for (int c = 0; c < C; ++c) {
       bits[c] = next[c];
       frac[c] += kFracStride;
       if (b + 1 < n_blocks) next[c] = load_frac<S>(frac[c]);
@@ -821,7 +822,8 @@ decode_kernel(const BatchArgs batch) {
   uint32_t *flag_sh = reinterpret_cast<uint32_t *>(smem + a.lut_bytes + 8 * 32 + 520);  // 4 words
   uint8_t *slots = smem + a.lut_bytes + 1024;
   const uint32_t bar = smem_u32(&bars[warp]);
-  const uint32_t buf_bytes = kChains * a.slot_bytes;
+  const uint32_t chains = (DOT || UPDATE) ? kChains : batch.item[ti].chains;
+  const uint32_t buf_bytes = chains * a.slot_bytes;
   const uint32_t slot0 = smem_u32(slots) + warp * bufs * buf_bytes;
   // per-warp ring for the packed fractions, behind all slots and their guard band
   const uint32_t ring =
@@ -852,14 +854,14 @@ decode_kernel(const BatchArgs batch) {
   const uint8_t *payload = a.container + a.pay_off;
   const uint32_t U = 32u * a.S;
   const uint32_t n_blocks = a.S >> 3;
-  uint32_t it, it_end;         // items left, in groups of kChains
+  uint32_t it, it_end;         // items left, in groups of `chains`
   {
     // groups_each for every warp and one more for the first groups_more of them, counted
     // across the CTAs first, so that every CTA gets its part of the longer runs
     const uint32_t me = warp * cta_count + cta_rank;
     const uint32_t each = batch.item[ti].groups_each, more = batch.item[ti].groups_more;
-    it = kChains * (each * me + (me < more ? me : more));
-    it_end = it + kChains * (each + (me < more ? 1u : 0u));
+    it = chains * (each * me + (me < more ? me : more));
+    it_end = it + chains * (each + (me < more ? 1u : 0u));
     if (it_end > a.n_work) it_end = a.n_work;
     if (warp >= n_warps) it = it_end = 0;
   }
@@ -889,6 +891,12 @@ decode_kernel(const BatchArgs batch) {
     if (at - win >= 32) load_window(at);
 #pragma unroll
     for (int c = 0; c < kChains; ++c) {
+      if (c && chains == 1) {
+        unit[c] = a.n_units;
+        pl[c].kind = kUnitSkip;
+        pl[c].word0 = pl[c].words = pl[c].copy_bytes = 0;
+        continue;
+      }
       const int k = (int)(at - win) + c;         // below 32: windows hold whole groups
       unit[c] = LIST ? __shfl_sync(0xFFFFFFFFu, my_unit, k) : (at + c < it_end ? at + c : a.n_units);
       pl[c].word0 = __shfl_sync(0xFFFFFFFFu, mine.word0, k);
@@ -943,13 +951,14 @@ decode_kernel(const BatchArgs batch) {
   };
   bool primed = false;         // the ring holds (or is receiving) the group's first fractions
   while (it < it_end) {
-    // Both units coded: decoded side by side as far as both have full blocks (all of them,
-    // but for the tensor's last unit).  Matrix-vector and update launches only take whole
-    // units this way.
+    // Both units (the one unit) coded: decoded side by side as far as both have full blocks
+    // (all of them, but for the tensor's last unit).  Matrix-vector and update launches only
+    // take whole units this way.
     bool pair = true;
     uint32_t common = n_blocks;
 #pragma unroll
     for (int c = 0; c < kChains; ++c) {
+      if (c && chains == 1) continue;
       pair = pair && pl[c].kind == kUnitCoded;
       if (real[c] >= a.full_units) {
         if (DOT || UPDATE || real[c] >= a.n_units) pair = false;
@@ -961,8 +970,12 @@ decode_kernel(const BatchArgs batch) {
 #pragma unroll
     for (int c = 0; c < kChains; ++c) fr[c] = MERGE ? frac_of(real[c]) : nullptr;
     if (MERGE) {
-      if (pair && !primed) ring_prologue<S>(ring, fr, common);
-      else if (!pair && primed) frac_wait<0>();
+      if (pair && !primed) {
+        if (chains == 1) ring_prologue<S, 1>(ring, fr, common);
+        else ring_prologue<S, kChains>(ring, fr, common);
+      } else if (!pair && primed) {
+        frac_wait<0>();
+      }
       primed = false;
     }
     if (staged) {
@@ -979,22 +992,23 @@ decode_kernel(const BatchArgs batch) {
     }
     const uint32_t slot = slot0 + buf * buf_bytes;
     LaneState st[kChains];
-    if (pair && !open_pair(pl, slot, a.slot_bytes, lenq, lane, st)) {
+    if (pair && !(chains == 1 ? open_unit(pl[0], slot, lenq, lane, st[0])
+                              : open_pair(pl, slot, a.slot_bytes, lenq, lane, st))) {
       pair = false;
       frac_wait<0>();          // the ring is used again
     }
     uint32_t out0[kChains];    // output element of the units' first elements
 #pragma unroll
-    for (int c = 0; c < kChains; ++c)
-      out0[c] = a.tile_cols ? __shfl_sync(0xFFFFFFFFu, my_out, (int)(it - win) + c) : real[c] * U;
+    for (int c = 0; c < kChains; ++c)      // (with one chain the second is not used)
+      out0[c] = a.tile_cols ? __shfl_sync(0xFFFFFFFFu, my_out, ((int)(it - win) + c) & 31) : real[c] * U;
 
     // The next group: copied into the other buffer now, where there is one (the whole group
     // then hides the latency of its copies), else brought into L2 and copied at the end.
     uint32_t nreal[kChains] = {a.n_units, a.n_units};
     UnitPlan npl[kChains];
-    const bool more = it + kChains < it_end;
+    const bool more = it + chains < it_end;
     if (more) {
-      take_group(it + kChains, nreal, npl);
+      take_group(it + chains, nreal, npl);
       if (bufs > 1) {
         staged = stage_units(a, npl, slot0 + (buf ^ 1) * buf_bytes, bar, lane);
       } else if (lane == 0) {
@@ -1007,8 +1021,8 @@ decode_kernel(const BatchArgs batch) {
     if (pair) {
       uint8_t *xb[kChains];
       const uint8_t *nfr[kChains] = {nullptr, nullptr};
-      if (MERGE && more && npl[0].copy_bytes && npl[1].copy_bytes && common == n_blocks &&
-          nreal[0] < a.full_units && nreal[1] < a.full_units) {
+      if (MERGE && more && npl[0].copy_bytes && (chains == 1 || npl[1].copy_bytes) &&
+          common == n_blocks && nreal[0] < a.full_units && (chains == 1 || nreal[1] < a.full_units)) {
 #pragma unroll
         for (int c = 0; c < kChains; ++c) nfr[c] = frac_of(nreal[c]);
       }
@@ -1022,12 +1036,21 @@ decode_kernel(const BatchArgs batch) {
           xb[c] = MERGE ? nullptr : a.out_exp + o;
           init_sink(sink, c, a, real[c], o, lane);
         }
-        if (lv.narrow && row_shift == kFastRow)
-          primed = decode_blocks_multi<S, MERGE, kFastRow>(st, lv, common, false, fr, nfr, sink, xb, ring);
-        else if (S != 7 && lv.narrow)            // kFastRow - 1, see narrow_rows
-          primed = decode_blocks_multi<S, MERGE, kFastRow - 1>(st, lv, common, false, fr, nfr, sink, xb, ring);
-        else
-          primed = decode_blocks_multi<S, MERGE, 0>(st, lv, common, canon, fr, nfr, sink, xb, ring);
+        if (DOT || UPDATE || chains == kChains) {
+          if (lv.narrow && row_shift == kFastRow)
+            primed = decode_blocks_multi<S, MERGE, kFastRow, kChains>(st, lv, common, false, fr, nfr, sink, xb, ring);
+          else if (S != 7 && lv.narrow)            // kFastRow - 1, see narrow_rows
+            primed = decode_blocks_multi<S, MERGE, kFastRow - 1, kChains>(st, lv, common, false, fr, nfr, sink, xb, ring);
+          else
+            primed = decode_blocks_multi<S, MERGE, 0, kChains>(st, lv, common, canon, fr, nfr, sink, xb, ring);
+        } else {
+          if (lv.narrow && row_shift == kFastRow)
+            primed = decode_blocks_multi<S, MERGE, kFastRow, 1>(st, lv, common, false, fr, nfr, sink, xb, ring);
+          else if (S != 7 && lv.narrow)
+            primed = decode_blocks_multi<S, MERGE, kFastRow - 1, 1>(st, lv, common, false, fr, nfr, sink, xb, ring);
+          else
+            primed = decode_blocks_multi<S, MERGE, 0, 1>(st, lv, common, canon, fr, nfr, sink, xb, ring);
+        }
         finish_sink(sink);
       };
       if (DOT) {
@@ -1052,21 +1075,20 @@ decode_kernel(const BatchArgs batch) {
         run(sink);
       }
       if (common == n_blocks) {
-        bool low = true;
-#pragma unroll
-        for (int c = 0; c < kChains; ++c) low = low && st[c].x == kStateLow;
+        bool low = st[0].x == kStateLow;
+        if (chains > 1) low = low && st[kChains - 1].x == kStateLow;
         if (__any_sync(0xFFFFFFFFu, !low) && lane == 0) raise(a.status, NZ_STATUS_BAD_STATE);
       } else if (!DOT && !UPDATE) {
 #pragma unroll 1
-        for (int c = 0; c < kChains; ++c) {
-          const int64_t delta = LIST ? ((int64_t)(it + c) - (int64_t)real[c]) * (int64_t)U : 0;
+        for (uint32_t c = 0; c < chains; ++c) {
+          const int64_t delta = LIST ? ((int64_t)(it + c) - (int64_t)(c ? real[1] : real[0])) * (int64_t)U : 0;
           LaneState one = c ? st[1] : st[0];
           decode_rest<S, MERGE>(a, one, c ? real[1] : real[0], common, delta, lv, canon, lane);
         }
       }
     } else {
 #pragma unroll 1
-      for (int c = 0; c < kChains; ++c) {
+      for (uint32_t c = 0; c < chains; ++c) {
         const uint32_t u = c ? real[1] : real[0];
         const UnitPlan p = c ? pl[1] : pl[0];
         if (DOT) {
@@ -1081,7 +1103,7 @@ decode_kernel(const BatchArgs batch) {
     }
     // every lane is done reading the slots
     __syncwarp();
-    it += kChains;
+    it += chains;
     if (it < it_end) {
       take_group(it, real, pl);
       if (bufs > 1) buf ^= 1;
