@@ -15,8 +15,10 @@
 //   [2560, 2576)         u32 misc[4]        (pad symbol, probability bits, -, -)
 // and in the whole-tensor compressor
 //   [1536, 3584)         u32 entries[256][2] (reciprocal, freq | cum << 16)
-//   [3584, 3600)         u32 misc[4]        (pad symbol, probability bits, finished
-//                                            histogram blocks, -)
+//   [0, 1024)            u32 chunk[256]     words of the units of a chunk, once the histogram
+//                                           has become the table
+//   [3584, 3616)         u32 misc[8]        (pad symbol, probability bits, finished histogram
+//                                            blocks, raw units, largest coded unit in words, -)
 //   [4096, 4096+4*(nu+1))           u32 unit_words[nu]  (bit 31 = raw)
 //   [.., + 64*nu)                   u16 lane_len[nu][32]   (words; 0 = unit raw)
 //   [.., + nu*32*cap*2)             u16 lane_words[nu][32][cap]   cap = lane_cap_words(S)
@@ -110,7 +112,7 @@ __device__ __forceinline__ uint32_t encoder_reciprocal(uint32_t freq) {
 }
 
 // Run by one block of 256 threads.
-__device__ __forceinline__ void normalize_block(const uint32_t *hist, uint16_t *freq,
+__device__ __forceinline__ void normalize_block(uint32_t *hist, uint16_t *freq,
                                                 uint32_t *enc_tab, uint2 *entries,
                                                 uint32_t *misc, uint16_t *container_freq,
                                                 uint32_t low_pb) {
@@ -122,6 +124,7 @@ __device__ __forceinline__ void normalize_block(const uint32_t *hist, uint16_t *
   const int t = threadIdx.x;  // 256 threads
   const int lane = t & 31, wid = t >> 5;
   const uint64_t h = __ldcg(hist + t);        // other blocks' atomics: not through L1
+  if (entries) hist[t] = 0;                   // the fused compressor's chunk sums start here
   // total count and number of distinct symbols
   uint64_t tot = h;
   uint32_t dis = h != 0;
@@ -244,7 +247,7 @@ __device__ __forceinline__ void normalize_block(const uint32_t *hist, uint16_t *
   }
 }
 __global__ void __launch_bounds__(256)
-normalize_kernel(const uint32_t *__restrict__ hist, uint16_t *__restrict__ freq,
+normalize_kernel(uint32_t *__restrict__ hist, uint16_t *__restrict__ freq,
                  uint32_t *__restrict__ enc_tab, uint2 *__restrict__ entries,
                  uint32_t *__restrict__ misc,
                  uint16_t *__restrict__ container_freq, uint32_t low_pb) {
@@ -371,6 +374,31 @@ encode_kernel(const uint8_t *__restrict__ sym, uint64_t n, uint32_t S, uint32_t 
   }
 }
 
+// Header, last offset and the zero bytes of the gaps (after the offset table and after the
+// payload), by one thread.
+__device__ __forceinline__ void write_header(uint8_t *container, uint64_t n, uint32_t S,
+                                             uint32_t n_units, uint32_t pb, uint64_t words,
+                                             uint32_t raw_units, uint32_t max_words) {
+  const uint64_t pay_off = payload_offset(n_units);
+  Header h;
+  h.magic = kMagic;
+  h.version = 1;
+  h.n_symbols = n;
+  h.lane_symbols = S;
+  h.len_quantum = len_quantum(S);
+  h.n_units = n_units;
+  h.prob_bits = pb;
+  h.payload_offset = pay_off;
+  h.payload_words = words;
+  h.total_bytes = align16(pay_off + words * 2);
+  h.n_raw_units = raw_units;
+  h.max_coded_unit_words = max_words;
+  *reinterpret_cast<Header *>(container) = h;
+  reinterpret_cast<uint32_t *>(container + kOffsetsOffset)[n_units] = (uint32_t)words;
+  for (uint64_t b = kOffsetsOffset + 4ull * (n_units + 1); b < pay_off; ++b) container[b] = 0;
+  for (uint64_t b = pay_off + words * 2; b < h.total_bytes; ++b) container[b] = 0;
+}
+
 // Exclusive scan of the unit sizes -> offset table in the container, plus the
 // header.  One block; the unit count is small (N / (32 S)).
 __global__ void __launch_bounds__(1024)
@@ -434,28 +462,7 @@ scan_kernel(const uint32_t *__restrict__ unit_words, uint32_t n_units, uint64_t 
   }
   __syncthreads();
   if (t == 0) {
-    const uint64_t run = part[32];
-    const uint32_t rr = raw_cnt[0], mm = max_w[0];
-    const uint64_t pay_off = payload_offset(n_units);
-    Header h;
-    h.magic = kMagic;
-    h.version = 1;
-    h.n_symbols = n;
-    h.lane_symbols = S;
-    h.len_quantum = len_quantum(S);
-    h.n_units = n_units;
-    h.prob_bits = misc[1];
-    h.payload_offset = pay_off;
-    h.payload_words = run;
-    h.total_bytes = align16(pay_off + run * 2);
-    h.n_raw_units = rr;
-    h.max_coded_unit_words = mm;
-    *reinterpret_cast<Header *>(container) = h;
-    uint32_t *offsets = reinterpret_cast<uint32_t *>(container + kOffsetsOffset);
-    offsets[n_units] = (uint32_t)run;
-    // zero the gaps: after the offset table and after the payload
-    for (uint64_t b = kOffsetsOffset + 4ull * (n_units + 1); b < pay_off; ++b) container[b] = 0;
-    for (uint64_t b = pay_off + run * 2; b < h.total_bytes; ++b) container[b] = 0;
+    write_header(container, n, S, n_units, misc[1], part[32], raw_cnt[0], max_w[0]);
   }
   uint64_t run = part[wid];
   uint32_t *offsets = reinterpret_cast<uint32_t *>(container + kOffsetsOffset);
@@ -588,7 +595,7 @@ int encode_exponents(const void *exp_in, uint64_t n, uint32_t S, void *container
   const uint32_t nu = (uint32_t)unit_count(n, S);
   int rc = histogram_u8(exp_in, n, sc + kScratchHist, st);
   if (rc) return rc;
-  normalize_kernel<<<1, 256, 0, st>>>((const uint32_t *)(sc + kScratchHist),
+  normalize_kernel<<<1, 256, 0, st>>>((uint32_t *)(sc + kScratchHist),
                                       (uint16_t *)(sc + kScratchFreq),
                                       (uint32_t *)(sc + kScratchTab), (uint2 *)nullptr,
                                       (uint32_t *)(sc + kScratchMisc),
@@ -743,6 +750,16 @@ bf16_histogram_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t *his
   }
 }
 
+// Clears the histogram and the counters.  A kernel and not a memset: a memset between two
+// kernels waits for the first and holds the second back (6 us of a 40 us compress), a kernel of
+// the chain hands over like the others.
+__global__ void __launch_bounds__(256) clear_kernel(uint32_t *hist, uint32_t *misc) {
+  dependent_trigger();
+  dependent_wait();
+  hist[threadIdx.x] = 0;
+  if (threadIdx.x < 8) misc[threadIdx.x] = 0;
+}
+
 // Matrix element behind stream element e (see the operand order in the decoder).
 __device__ __forceinline__ uint64_t source_index(uint64_t e, uint32_t cols) {
   if (!cols) return e;
@@ -751,6 +768,13 @@ __device__ __forceinline__ uint64_t source_index(uint64_t e, uint32_t cols) {
   const uint32_t spr = cols >> 6;
   const uint64_t g = block / spr;
   const uint32_t kb = (uint32_t)(block - g * spr);
+  return (4 * g + (w >> 6)) * cols + kb * 64u + (w & 63u);
+}
+
+__device__ __forceinline__ uint32_t source_index32(uint32_t e, uint32_t cols) {
+  if (!cols) return e;
+  const uint32_t block = e >> 8, w = e & 255u, spr = cols >> 6;
+  const uint32_t g = block / spr, kb = block - g * spr;
   return (4 * g + (w >> 6)) * cols + kb * 64u + (w & 63u);
 }
 
@@ -985,8 +1009,8 @@ __device__ __forceinline__ void encode_blocks(const uint16_t *__restrict__ src, 
 template <int S>
 __global__ void __launch_bounds__(kFusedWarps * 32)
 bf16_encode_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uint32_t n_units,
-                   uint32_t cols, const uint2 *__restrict__ entries,
-                   const uint32_t *__restrict__ misc, uint32_t cap_s, uint32_t out_words,
+                   uint32_t cols, const uint2 *__restrict__ entries, uint32_t *misc,
+                   uint32_t *chunk, uint32_t chunk_lg, uint32_t cap_s, uint32_t out_words,
                    uint8_t *__restrict__ frac_out, uint32_t *__restrict__ unit_words,
                    uint8_t *__restrict__ slots, uint32_t slot_stride) {
   extern __shared__ __align__(16) uint8_t enc_smem[];
@@ -1005,7 +1029,7 @@ bf16_encode_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uin
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t lenq = len_quantum(LS);
   const uint32_t cap = lane_cap_words(LS);
-  const uint64_t U = 32ull * LS;
+  const uint32_t U = 32u * LS;
   // a warp's cell: 16 words of lane lengths, then 32 slices of cap_s words one word apart;
   // behind it the place where the unit takes its final form
   const uint32_t sstride = cap_s + 1;
@@ -1021,15 +1045,15 @@ bf16_encode_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uin
   for (uint32_t u = blockIdx.x * n_warps + warp; u < n_units; u += gridDim.x * n_warps) {
     // the next kernel of the pipeline may be set up while the last units are coded
     if (u + gridDim.x * n_warps >= n_units) dependent_trigger();
-    const uint64_t first = (uint64_t)u * U;
-    const uint64_t count = (n - first < U) ? (n - first) : U;
+    const uint32_t first = u * U;                      // element indices are below 2^32
+    const uint32_t left = (uint32_t)n - first, count = left < U ? left : U;
     uint32_t x = kStateLow, pos = top, spilled = 0;
     if (count == U) {
       // whole units walk two pointers down, block by block (in operand order a unit's blocks
       // are 64 elements apart in the lane's row; otherwise 256)
-      const uint64_t e_last = first + (uint64_t)(n_blocks - 1) * 256 + lane * 8;
-      const uint16_t *src = in + source_index(e_last, cols);
-      uint8_t *fdst = frac_out + e_last * (S + 1) / 8;
+      const uint32_t e_last = first + (n_blocks - 1) * 256 + lane * 8;
+      const uint16_t *src = in + source_index32(e_last, cols);
+      uint8_t *fdst = frac_out + ((uint64_t)e_last * (S + 1) >> 3);
       const uint32_t step = cols ? 64u : 256u;
       if (big)
         encode_blocks<S, true>(src, step, fdst, n_blocks, tab, pow_m, top, limit, x, pos, spilled);
@@ -1040,7 +1064,8 @@ bf16_encode_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uin
 #pragma unroll 1
       for (int32_t blk = (int32_t)n_blocks - 1; blk >= 0; --blk) {
         uint32_t lo, hi;
-        load_group<S>(in, first + (uint64_t)blk * 256 + lane * 8, n, cols, pad, frac_out, true, lo, hi);
+        load_group<S>(in, (uint64_t)first + (uint64_t)blk * 256 + lane * 8, n, cols, pad, frac_out, true,
+                      lo, hi);
         if (pos < limit) {
           spilled += (top - pos) >> 1;
           pos = top;
@@ -1060,10 +1085,17 @@ bf16_encode_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uin
       if (lane >= (uint32_t)o) incl += v;
     }
     const uint32_t total = 16u + __shfl_sync(0xFFFFFFFFu, incl, 31);
-    const uint64_t raw_words = (count + 1) / 2;
+    const uint32_t raw_words = (count + 1) / 2;
     const bool too_long = __any_sync(0xFFFFFFFFu, words > cap);       // the format's own limit
     const bool raw = too_long || total >= raw_words;
-    if (lane == 0) unit_words[u] = raw ? ((uint32_t)raw_words | kRawFlag) : total;
+    if (lane == 0) {
+      unit_words[u] = raw ? (raw_words | kRawFlag) : total;
+      if (chunk) {
+        atomicAdd(chunk + (u >> chunk_lg), raw ? raw_words : total);
+        if (raw) atomicAdd(misc + 3, 1u);
+        else atomicMax(misc + 4, total);
+      }
+    }
     if (raw) continue;                  // placed from the input by place_units_kernel
     uint16_t *slot = reinterpret_cast<uint16_t *>(slots + (uint64_t)u * slot_stride);
     if (__any_sync(0xFFFFFFFFu, spilled != 0)) {
@@ -1134,22 +1166,58 @@ bf16_encode_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uin
 }
 
 // Every unit to its place in the payload: coded units from their slots, raw units
-// (exponent bytes as they are) from the input.
+// (exponent bytes as they are) from the input.  A block has `per` consecutive units.  Unless
+// scan_kernel has written the offset table (chunk == null), the block finds where its units
+// start by itself -- the sums of the chunks before its chunk and of the units before its first
+// in the chunk, some hundred words -- and writes their part of the table; the last block
+// writes the header.  (The scan as a kernel of its own took 3 us for 4096 units and 11 us for
+// 28 thousand.)
 template <int S>
 __global__ void __launch_bounds__(128)
 place_units_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uint32_t n_units,
-                   uint32_t cols, const uint8_t *__restrict__ slots, uint32_t slot_stride,
-                   uint8_t *__restrict__ container) {
+                   uint32_t cols, const uint32_t *__restrict__ unit_words,
+                   const uint32_t *__restrict__ chunk, uint32_t chunk_lg,
+                   const uint32_t *__restrict__ misc, uint32_t per,
+                   const uint8_t *__restrict__ slots, uint32_t slot_stride, uint8_t *container) {
+  __shared__ uint32_t part[4];
   dependent_wait();
-  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t U = 32ull * LS;
-  const uint32_t *offsets = reinterpret_cast<const uint32_t *>(container + kOffsetsOffset);
+  uint32_t *offsets = reinterpret_cast<uint32_t *>(container + kOffsetsOffset);
   uint16_t *payload = reinterpret_cast<uint16_t *>(container + payload_offset(n_units));
-  for (uint32_t u = blockIdx.x * 4 + (threadIdx.x >> 5); u < n_units; u += gridDim.x * 4) {
-    const uint32_t off = offsets[u];
-    const uint32_t w0 = off & ~kRawFlag;
+  const uint32_t u0 = blockIdx.x * per;
+  // this lane's unit of the block, its size word and where it starts
+  const uint32_t mine = u0 + lane < n_units && lane < per ? unit_words[u0 + lane] : 0u;
+  uint32_t start = 0;
+  if (chunk) {
+    const uint32_t c0 = u0 >> chunk_lg, in_chunk = u0 & ((1u << chunk_lg) - 1u);
+    uint32_t sum = 0;
+    for (uint32_t i = threadIdx.x; i < c0; i += 128) sum += chunk[i];
+    for (uint32_t i = threadIdx.x; i < in_chunk; i += 128)
+      sum += unit_words[(c0 << chunk_lg) + i] & ~kRawFlag;
+    sum = __reduce_add_sync(0xFFFFFFFFu, sum);
+    if (lane == 0) part[warp] = sum;
+    __syncthreads();
+    const uint32_t before = part[0] + part[1] + part[2] + part[3];    // below 2^31 words
+    uint32_t incl = mine & ~kRawFlag;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= (uint32_t)o) incl += v;
+    }
+    start = before + incl - (mine & ~kRawFlag);
+    if (warp == 0 && lane < per && u0 + lane < n_units) offsets[u0 + lane] = start | (mine & kRawFlag);
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 31)
+      write_header(container, n, LS, n_units, misc[1], before + incl, misc[3], misc[4]);
+  } else if (u0 + lane < n_units && lane < per) {
+    start = offsets[u0 + lane] & ~kRawFlag;
+  }
+  for (uint32_t j = warp; j < per; j += 4) {
+    const uint32_t u = u0 + j;
+    if (u >= n_units) break;
+    const uint32_t size = __shfl_sync(0xFFFFFFFFu, mine, j), w0 = __shfl_sync(0xFFFFFFFFu, start, j);
     uint16_t *dst = payload + w0;
-    if (off & kRawFlag) {
+    if (size & kRawFlag) {
       const uint64_t first = (uint64_t)u * U;
       const uint64_t count = (n - first < U) ? (n - first) : U;
       uint8_t *d8 = reinterpret_cast<uint8_t *>(dst);
@@ -1158,7 +1226,7 @@ place_units_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uin
       if ((count & 1) && lane == 0) d8[count] = 0;
       continue;
     }
-    const uint32_t words = (offsets[u + 1] & ~kRawFlag) - w0;
+    const uint32_t words = size;
     const uint32_t *src = reinterpret_cast<const uint32_t *>(slots + (uint64_t)u * slot_stride);
     // 32-bit stores; when the destination starts on an odd word, one 16-bit store first and
     // then source words shifted by half a word.  The copy is bound by the latency of its
@@ -1235,11 +1303,10 @@ static int compress_fused(const void *in, uint64_t n, uint32_t LS, uint32_t cols
   uint8_t *sc = (uint8_t *)scratch;
   uint8_t *cont = (uint8_t *)container;
   const uint32_t nu = (uint32_t)unit_count(n, LS);
-  // histogram, tables (overwritten) and the count of finished histogram blocks
-  NZ_CUDA_TRY(cudaMemsetAsync(sc + kScratchHist, 0, kFusedMisc + 16, st));
   uint32_t *hist = (uint32_t *)(sc + kScratchHist), *misc = (uint32_t *)(sc + kFusedMisc);
   uint2 *entries = (uint2 *)(sc + kScratchTab);
   uint16_t *freq = (uint16_t *)(sc + kScratchFreq), *cont_freq = (uint16_t *)(cont + kFreqOffset);
+  NZ_CUDA_TRY(launch_dependent(clear_kernel, 1, 256, 0, st, hist, misc));
   if (n) {
     uint64_t blocks = (n / 8 + kHistThreads - 1) / kHistThreads;
     const uint64_t capb = (uint64_t)sm_count() * 8;
@@ -1249,9 +1316,14 @@ static int compress_fused(const void *in, uint64_t n, uint32_t LS, uint32_t cols
                                  (const uint16_t *)in, n, hist, misc + 2, freq, entries, misc,
                                  cont_freq, low_pb));
   } else {
-    NZ_CUDA_TRY(launch_dependent(normalize_kernel, 1, 256, 0, st, (const uint32_t *)hist, freq,
+    NZ_CUDA_TRY(launch_dependent(normalize_kernel, 1, 256, 0, st, hist, freq,
                                  (uint32_t *)nullptr, entries, misc, cont_freq, low_pb));
   }
+  // chunks of the units' sizes: 256 sums at most, and chunks of at most 512 units (a block of
+  // the placement adds up its chunk); more units than that are scanned by a kernel
+  uint32_t chunk_lg = 0;
+  while (((uint64_t)nu >> chunk_lg) > 255) ++chunk_lg;
+  uint32_t *chunk = nu && chunk_lg <= 9 ? hist : nullptr;
   if (nu) {
     const uint32_t cell_words = (16 + 32 * (L.cap_s + 1) + 7) & ~7u;
     const uint32_t warp_bytes = (cell_words + L.out_words) * 2;
@@ -1282,19 +1354,21 @@ static int compress_fused(const void *in, uint64_t n, uint32_t LS, uint32_t cols
     const uint32_t capb = (uint32_t)sm_count() * per_sm;
     if (blocks > capb) blocks = capb;
     NZ_CUDA_TRY(launch_dependent(kern, blocks, warps * 32, smem, st, (const uint16_t *)in, n, LS, nu,
-                                 cols, (const uint2 *)entries, (const uint32_t *)misc, L.cap_s, L.out_words,
+                                 cols, (const uint2 *)entries, misc, chunk, chunk_lg, L.cap_s, L.out_words,
                                  (uint8_t *)frac_out, (uint32_t *)(sc + L.unit_words),
                                  sc + L.slots, L.slot_stride));
   }
-  NZ_CUDA_TRY(launch_dependent(scan_kernel, 1, 1024, 0, st, (const uint32_t *)(sc + L.unit_words),
-                               nu, n, LS, (const uint32_t *)misc, cont));
+  if (!chunk)
+    NZ_CUDA_TRY(launch_dependent(scan_kernel, 1, 1024, 0, st, (const uint32_t *)(sc + L.unit_words),
+                                 nu, n, LS, (const uint32_t *)misc, cont));
   if (nu) {
-    uint32_t blocks = (nu + 3) / 4;
-    const uint32_t capb = (uint32_t)sm_count() * 16;
-    if (blocks > capb) blocks = capb;
-    NZ_CUDA_TRY(launch_dependent(place_units_kernel<S>, blocks, 128, 0, st, (const uint16_t *)in,
-                                 n, LS, nu, cols, (const uint8_t *)(sc + L.slots), L.slot_stride,
-                                 cont));
+    // a unit per warp while that leaves blocks to spare, four on large tensors (less to add up)
+    const uint32_t per = nu <= 8192 ? 4 : 16;
+    NZ_CUDA_TRY(launch_dependent(place_units_kernel<S>, (nu + per - 1) / per, 128, 0, st,
+                                 (const uint16_t *)in, n, LS, nu, cols,
+                                 (const uint32_t *)(sc + L.unit_words), (const uint32_t *)chunk, chunk_lg,
+                                 (const uint32_t *)misc, per, (const uint8_t *)(sc + L.slots),
+                                 L.slot_stride, cont));
   }
   return NZ_OK;
 }

@@ -42,8 +42,10 @@ def test_encoder_branches(s, kind):
             assert np.array_equal(frac.cpu().numpy(), f_ref), (s, kind, S, n)
 
 
-def test_many_units_per_warp():
-    n = 32 * 8 * 148 * 48 * 3 + 1001
+@pytest.mark.parametrize("units", (255, 256, 257, 148 * 48 * 3 + 4, 255 * 512 + 1))
+def test_many_units(units):
+    # chunks of one and more units, several units per warp, and offsets from the scan kernel
+    n = 256 * units - 23
     bits = bits_of("peaked", n, 3)
     cont, frac, _ = A.compress(A.from_bits(bits), 7, 8)
     c_ref, f_ref = O.compress_bf16(bits, 7, 8)
