@@ -171,9 +171,15 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
         ++now[hi];
       }
     }
+    // the table has to be written first: 16 bytes per lane and store, by the few warps that a
+    // small launch has
     uint64_t worst = 0;
-    for (uint32_t t = 0; t < count; ++t)
-      if (cost(t, now[t]) > worst) worst = cost(t, now[t]);
+    for (uint32_t t = 0; t < count; ++t) {
+      const uint64_t own = (work_units(items[t]) + now[t] - 1) / now[t];
+      const uint32_t writers = own < 4 && own < cap[t] ? (uint32_t)own : 4;
+      const uint64_t c = cost(t, now[t]) + (4096u << sh) / (16 * writers);
+      if (c > worst) worst = c;
+    }
     if (worst < best) {
       best = worst;
       b.lut_shift = sh;

@@ -648,17 +648,17 @@ int encode_exponents(const void *exp_in, uint64_t n, uint32_t S, void *container
 // Replaces split + nvcomp compress + right-sizing of the reference's write path
 // (cuda/high_level.cu:81-124) in two sweeps over the bf16 input:
 //   1. bf16_histogram_kernel  counts the exponent bytes (after the rounding of the
-//      lossy precisions, exactly as the split computes them);
+//      lossy precisions, exactly as the split computes them) and makes the frequency table;
 //   2. bf16_encode_kernel     reads the input again (largely from L2 for tensors of
 //      the usual size), writes the packed fractions and rANS-codes the exponents.
-//      A warp codes one unit at a time (two side by side measured slower: the hardware interleaves warps better than the compiler interleaves the chains of
-//      one warp, and a warp's cells then take half the shared memory); each lane's 16-bit
-//      words go into its slice of a shared-memory cell, the
-//      cell is then squeezed into the unit's final layout and written with
-//      coalesced stores into the unit's slot of the scratch area.
-// scan_kernel then fixes the offsets and place_units_kernel copies every slot to
-// its place in the payload.  The input may be a matrix to be stored in operand
-// order: the element a lane handles is then found through operand_index().
+//      A warp codes one unit at a time (two side by side measured slower: the hardware
+//      interleaves warps better than the compiler interleaves the chains of one warp);
+//      each lane's 16-bit words go into its slice of a shared-memory cell, the lanes then
+//      move their streams into the unit's final layout, which is written with coalesced
+//      stores into the unit's slot of the scratch area.
+// place_units_kernel copies every slot to its place in the payload and writes offsets and
+// header.  The input may be a matrix to be stored in operand order: the element a lane
+// handles is then found through source_index().
 // The results are byte-identical to split + nz_encode_exponents.
 //
 // A lane's slice holds `cap_s` words (4 bits per symbol on average; real weights
