@@ -52,8 +52,9 @@ class _Entry:
     # completed the entry is settled: right-sized container, real max_unit_words.
     pending: Optional[tuple] = None
     version: int = 0          # bumped when the container tensor is replaced
-    # (argument block of a single decode, its address): struct nz_decompress_item, which the
-    # library only reads; built at the first read of these bytes
+    # (argument block of a single decode, its address, the container it describes): struct
+    # nz_decompress_item, which the library only reads; built at the first read of these bytes,
+    # good only as long as `container` is that very tensor
     item: Optional[tuple] = None
 
 
@@ -350,7 +351,7 @@ class CodecBackend:
         entry.max_unit_words = words.value
         entry.container = entry.container[:total.value].clone()     # enqueued after the write
         entry.version += 1
-        entry.item = None           # described the buffer that has just been replaced
+        entry.item = None           # describes the buffer that has just been replaced
 
     def settle_all(self) -> None:
         """Wait for every write still in flight and right-size its container (for instance
@@ -393,7 +394,9 @@ class CodecBackend:
     def _decode(self, entry: _Entry, out: torch.Tensor) -> None:
         # the per-call flag is the promise that the compressed bytes are not fresh, which lets
         # this launch set up while the previous kernel of the stream drains
-        item = entry.item or self._describe(entry)
+        item = entry.item
+        if item is None or item[2] is not entry.container:
+            item = self._describe(entry)
         rc = self._lib.nz_decompress_bf16_item(
             item[1], out.data_ptr(),
             _lib.NZ_ITEM_INPUTS_STABLE if entry.stamp < _next_op() - 1 else 0,
@@ -402,17 +405,20 @@ class CodecBackend:
             _lib.check(rc)
 
     def _describe(self, entry: _Entry):
-        """The entry's argument block for the library, filled before it is published."""
+        """The entry's argument block for the library, filled before it is published.  Another
+        thread may settle the entry meanwhile: the block names the container it describes,
+        which keeps that buffer alive and lets the next read see that it was replaced."""
+        container = entry.container
         item = _lib.DecompressItem()
-        item.container = _ptr(entry.container)
-        item.container_bytes = entry.container.numel()
+        item.container = _ptr(container)
+        item.container_bytes = container.numel()
         item.frac_in = _ptr(entry.fractions)
         item.n = entry.numel
         item.max_unit_words = entry.max_unit_words
         item.operand_cols = entry.operand_cols
         item.lane_symbols = entry.lane_symbols
         self._set_normalizer(item, entry)
-        entry.item = described = (item, ctypes.addressof(item))
+        entry.item = described = (item, ctypes.addressof(item), container)
         return described
 
     def read_rows(self, name: str, rows: torch.Tensor, row_len: int) -> torch.Tensor:
