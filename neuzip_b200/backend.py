@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import enum
 import functools
+import threading
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence
 
@@ -77,12 +78,13 @@ def _stable_flag(entries, op: int) -> int:
 
 class _Batch:
     """Argument blocks of a batched decode, rebuilt when an entry is replaced."""
-    __slots__ = ("names", "outs", "entries", "versions", "blocks", "lane_symbols")
+    __slots__ = ("names", "outs", "entries", "containers", "versions", "blocks", "lane_symbols")
 
     def __init__(self, names, outs) -> None:
         self.names = list(names)
         self.outs = list(outs)
         self.entries = []
+        self.containers = []
         self.versions = []
         self.blocks = None
         self.lane_symbols = 0
@@ -173,7 +175,9 @@ class CodecBackend:
         # (nz_linear_bf16) on operand-order weights; 0 = always decode, then library GEMM
         self.fused_linear_max_rows = 0
         self._lin_ws: Optional[torch.Tensor] = None
-        # pinned header slots and events of writes that have not been right-sized yet
+        # pinned header slots and events of writes that have not been right-sized yet; the
+        # lock covers the pools and the step from `pending` to settled
+        self._pending_lock = threading.RLock()
         self._hdr_chunks: List[torch.Tensor] = []
         self._hdr_base: List[int] = []
         self._hdr_free: List[int] = []
@@ -286,8 +290,9 @@ class CodecBackend:
         cap = int(L.nz_container_bound(n, S))
         staging = torch.empty(cap, dtype=torch.uint8, device="cuda")
         scratch = self._scratch_for(int(L.nz_adamw_compressed_scratch_bytes(n, S)))
+        container = entry.container      # kept until the launch is enqueued
         _lib.check(L.nz_adamw_compressed_bf16(
-            _ptr(entry.container), entry.container.numel(), _ptr(entry.fractions), n,
+            _ptr(container), container.numel(), _ptr(entry.fractions), n,
             entry.operand_cols, self.precision, S, entry.max_unit_words, int(self.canonical_nan),
             _ptr(grad), _ptr(exp_avg), _ptr(exp_avg_sq), lr, beta1, beta2, eps, weight_decay, step,
             grad_scale, _ptr(frac), _ptr(staging), cap, _ptr(scratch), scratch.numel(),
@@ -305,14 +310,15 @@ class CodecBackend:
         after that copy has completed.  `sync_writes = True` restores the blocking form.
         Header slots (one pinned buffer, 64 bytes each) and events are pooled: a write
         allocates no pinned memory and creates no event once the pools are warm."""
-        if replaced is not None and replaced.pending is not None:
-            # overwritten before it was ever settled: its slot and event go back (a copy
-            # still in flight into the slot lands before the next one, same stream)
-            self._release_pending(replaced)
-        if not self._hdr_free:
-            self._grow_header_pool()
-        slot = self._hdr_free.pop()
-        event = self._event_pool.pop() if self._event_pool else torch.cuda.Event()
+        with self._pending_lock:
+            if replaced is not None:
+                # overwritten before it was ever settled: its slot and event go back (a copy
+                # still in flight into the slot lands before the next one, same stream)
+                self._release_pending(replaced)
+            if not self._hdr_free:
+                self._grow_header_pool()
+            slot = self._hdr_free.pop()
+            event = self._event_pool.pop() if self._event_pool else torch.cuda.Event()
         _lib.check(self._lib.nz_container_header_async(
             _ptr(entry.container), self._hdr_base[slot >> 8] + 64 * (slot & 255), _stream()))
         event.record()
@@ -329,29 +335,37 @@ class CodecBackend:
         self._hdr_free.extend(range(256 * index + 255, 256 * index - 1, -1))
 
     def _release_pending(self, entry: _Entry) -> None:
-        slot, event = entry.pending
-        self._hdr_free.append(slot)
-        self._event_pool.append(event)
-        entry.pending = None
+        """Slot and event of an entry that will not be settled (any more) go back, once."""
+        with self._pending_lock:
+            if entry.pending is not None:
+                slot, event = entry.pending
+                entry.pending = None
+                self._hdr_free.append(slot)
+                self._event_pool.append(event)
 
     def _settle(self, entry: _Entry, block: bool) -> None:
-        if entry.pending is None:
+        pending = entry.pending
+        if pending is None:
             return
-        slot, event = entry.pending
+        slot, event = pending
         if block:
-            event.synchronize()
+            event.synchronize()              # outside the lock: other entries may be settled
         elif not event.query():
             return
-        total, words = ctypes.c_uint64(0), ctypes.c_uint32(0)
-        rc = self._lib.nz_parse_header(self._hdr_base[slot >> 8] + 64 * (slot & 255),
-                                       ctypes.byref(total), ctypes.byref(words))
-        self._release_pending(entry)
-        if rc:
-            raise _lib.NeuzipError("write produced no NZR1 container")
-        entry.max_unit_words = words.value
-        entry.container = entry.container[:total.value].clone()     # enqueued after the write
-        entry.version += 1
-        entry.item = None           # describes the buffer that has just been replaced
+        with self._pending_lock:
+            if entry.pending is not pending:
+                return                       # another thread has settled or replaced it meanwhile
+            total, words = ctypes.c_uint64(0), ctypes.c_uint32(0)
+            rc = self._lib.nz_parse_header(self._hdr_base[slot >> 8] + 64 * (slot & 255),
+                                           ctypes.byref(total), ctypes.byref(words))
+            self._release_pending(entry)
+            if rc:
+                raise _lib.NeuzipError("write produced no NZR1 container")
+            # a reader that sees the new container also sees its largest unit
+            entry.max_unit_words = words.value
+            entry.container = entry.container[:total.value].clone()     # enqueued after the write
+            entry.version += 1
+            entry.item = None       # describes the buffer that has just been replaced
 
     def settle_all(self) -> None:
         """Wait for every write still in flight and right-size its container (for instance
@@ -453,8 +467,9 @@ class CodecBackend:
         L = self._lib
         scratch_bytes = int(L.nz_gather_scratch_bytes(k, row_len, entry.lane_symbols))
         scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=_CUDA)
+        container = entry.container      # kept until the launch is enqueued
         _lib.check(L.nz_gather_rows_normalized_bf16(
-            _ptr(entry.container), entry.container.numel(), _ptr(entry.fractions), entry.numel,
+            _ptr(container), container.numel(), _ptr(entry.fractions), entry.numel,
             self.precision, entry.lane_symbols, entry.max_unit_words, int(self.canonical_nan),
             row_len, _ptr(rows), k, _ptr(entry.normalizers),
             self.normalizer_size if entry.normalizers is not None else 0, _ptr(out), _ptr(scratch),
@@ -487,9 +502,10 @@ class CodecBackend:
         if entries:
             items = (_lib.DecompressItem * len(entries))()
             flags = _stable_flag(entries, _next_op())
-            for k, e in enumerate(entries):
-                items[k].container = _ptr(e.container)
-                items[k].container_bytes = e.container.numel()
+            containers = [e.container for e in entries]     # kept until the launch is enqueued
+            for k, (e, container) in enumerate(zip(entries, containers)):
+                items[k].container = _ptr(container)
+                items[k].container_bytes = container.numel()
                 items[k].frac_in = _ptr(e.fractions)
                 items[k].n = e.numel
                 items[k].max_unit_words = e.max_unit_words
@@ -518,16 +534,19 @@ class CodecBackend:
         entries = [self._cache[n] for n in batch.names]
         for e in entries:
             self._settle(e, block=False)
+        # taken before the pointers: an entry that another thread settles meanwhile is bound anew
+        versions = [e.version for e in entries]
+        containers = [e.container for e in entries]
         # two argument blocks: with and without the promise that the inputs are stable
         blocks = []
         for flags in (0, _lib.NZ_ITEM_INPUTS_STABLE):
             items = (_lib.DecompressItem * len(entries))()
-            for k, (e, out) in enumerate(zip(entries, batch.outs)):
+            for k, (e, container, out) in enumerate(zip(entries, containers, batch.outs)):
                 if out.numel() < e.numel or out.dtype != torch.bfloat16 or not out.is_cuda:
                     raise ValueError(
                         "output buffers must be CUDA bf16 tensors of at least numel elements")
-                items[k].container = _ptr(e.container)
-                items[k].container_bytes = e.container.numel()
+                items[k].container = _ptr(container)
+                items[k].container_bytes = container.numel()
                 items[k].frac_in = _ptr(e.fractions)
                 items[k].n = e.numel
                 items[k].max_unit_words = e.max_unit_words
@@ -537,16 +556,17 @@ class CodecBackend:
                 items[k].lane_symbols = e.lane_symbols
                 self._set_normalizer(items[k], e)
             blocks.append(items)
-        # the entries keep their tensors alive as long as the batch refers to them
+        # the batch keeps the tensors it names alive
         batch.entries, batch.blocks, batch.lane_symbols = entries, blocks, entries[0].lane_symbols
-        batch.versions = [e.version for e in entries]
+        batch.containers, batch.versions = containers, versions
 
     def run_batch(self, batch: _Batch) -> None:
         cache = self._cache
         for name, entry, version in zip(batch.names, batch.entries, batch.versions):
+            pending = entry.pending
             # written, imported or erased since -- or its write has settled meanwhile
             if (cache.get(name) is not entry or entry.version != version
-                    or (entry.pending is not None and entry.pending[1].query())):
+                    or (pending is not None and pending[1].query())):
                 self._bind_batch(batch)
                 break
         items = batch.blocks[1 if _stable_flag(batch.entries, _next_op()) else 0]
@@ -642,8 +662,9 @@ class CodecBackend:
             turn, group, before = reducer.next_set()
             after = ctypes.c_uint32(0)
             _next_op()
+            container = entry.container      # kept until the launch is enqueued
             rc = L.nz_linear_allreduce_bf16(
-                _ptr(entry.container), entry.container.numel(), _ptr(entry.fractions), out_f, in_f,
+                _ptr(container), container.numel(), _ptr(entry.fractions), out_f, in_f,
                 self.precision, entry.lane_symbols, entry.max_unit_words, int(self.canonical_nan),
                 _ptr(x), m, _ptr(bias.contiguous() if bias is not None else None), _ptr(y),
                 ctypes.byref(group), before, ctypes.byref(after), _ptr(self._status), _stream())
@@ -658,8 +679,9 @@ class CodecBackend:
         if self._lin_ws is None or self._lin_ws.numel() < need:
             self._lin_ws = torch.empty(need, dtype=torch.uint8, device="cuda")
         _next_op()
+        container = entry.container      # kept until the launch is enqueued
         rc = L.nz_linear_bf16(
-            _ptr(entry.container), entry.container.numel(), _ptr(entry.fractions), out_f, in_f,
+            _ptr(container), container.numel(), _ptr(entry.fractions), out_f, in_f,
             self.precision, entry.lane_symbols, entry.max_unit_words, int(self.canonical_nan),
             _ptr(x), m, _ptr(bias.contiguous() if bias is not None else None), _ptr(y),
             _ptr(self._lin_ws), self._lin_ws.numel(), _ptr(self._status), _stream())
@@ -703,8 +725,9 @@ class CodecBackend:
             scratch = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
             self._vec_scratch[(entry.numel, in_f)] = scratch
         scratch_bytes = scratch.numel()
+        container = entry.container      # kept until the launch is enqueued
         _lib.check(L.nz_linear_vec_bf16(
-            _ptr(entry.container), entry.container.numel(), _ptr(entry.fractions), entry.numel,
+            _ptr(container), container.numel(), _ptr(entry.fractions), entry.numel,
             self.precision, entry.lane_symbols, entry.max_unit_words, int(self.canonical_nan),
             in_f, _ptr(self._vec_x), _ptr(bias.contiguous() if bias is not None else None),
             _ptr(y), _ptr(scratch), scratch_bytes, _ptr(self._status), _stream()))
@@ -752,7 +775,7 @@ class CodecBackend:
         if normalizers is not None:
             normalizers = normalizers.to(device="cuda", dtype=torch.uint8).contiguous()
         replaced = self._cache.get(name)
-        if replaced is not None and replaced.pending is not None:
+        if replaced is not None:
             self._release_pending(replaced)
         self._cache[name] = _Entry(n, torch.bfloat16, int(blob["lane_symbols"]),
                                    int(blob["max_unit_words"]), container, fractions, normalizers,
@@ -761,7 +784,7 @@ class CodecBackend:
     # -- extras -----------------------------------------------------------
     def erase(self, name: str) -> None:
         gone = self._cache.pop(name, None)
-        if gone is not None and gone.pending is not None:
+        if gone is not None:
             self._release_pending(gone)
 
     def entry(self, name: str) -> _Entry:

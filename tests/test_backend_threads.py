@@ -1,8 +1,6 @@
 """What two threads may do to one stored tensor, forced on the CPU by running the second
-thread's step at the point where it hurts most: a description of a container that is published
-after the container has been replaced."""
-import ctypes
-
+thread's step at the point where it hurts most: a container replaced while a description of it
+is made, and a write settled, replaced or erased while another thread settles it."""
 import torch
 
 from neuzip_b200 import _lib, backend
@@ -72,3 +70,51 @@ def test_description_published_after_the_container_was_replaced(monkeypatch):
     for _ in range(2):
         be._decode(entry, out)
         assert be._lib.seen[-1] == described(entry)
+
+
+def test_two_threads_settle_one_entry(monkeypatch):
+    be, entry = make(monkeypatch)
+    # the other thread settles while this one asks whether the header has arrived
+    entry.pending[1].on_query = lambda: be._settle(entry, block=False)
+    be._settle(entry, block=False)
+    assert be._hdr_free == [3] and len(be._event_pool) == 1       # given back once
+    assert entry.pending is None and entry.version == 1 and entry.container.numel() == 64
+
+
+def test_replaced_while_settled(monkeypatch):
+    be, entry = make(monkeypatch)
+    entry.pending[1].on_query = lambda: be.erase("w")
+    be._settle(entry, block=True)
+    assert be._hdr_free == [3] and len(be._event_pool) == 1
+
+
+def test_batch_bound_while_an_entry_is_settled(monkeypatch):
+    be, entry = make(monkeypatch)
+    pending = entry.pending
+    entry.pending = None
+    entry.stamp = 1 << 60                   # a fresh write: the batch runs the block it fills first
+    fill = be._set_normalizer
+
+    def settled_by_another_thread(item, e):
+        if be._set_normalizer is not fill:
+            be._set_normalizer = fill
+            e.pending = pending
+            be._settle(e, block=True)
+        fill(item, e)
+
+    class Out:                               # make_batch wants CUDA outputs
+        dtype, is_cuda = torch.bfloat16, True
+        numel = staticmethod(lambda: 16)
+        data_ptr = staticmethod(lambda: 0)
+
+    be._set_normalizer = settled_by_another_thread
+    batch = be.make_batch(["w"], [Out()])
+    seen = []
+
+    def batched(items, count, precision, lane, canon, status, stream):
+        seen.append((items[0].container, items[0].container_bytes, items[0].max_unit_words))
+        return 0
+
+    be._lib.nz_decompress_bf16_batch = batched
+    be.run_batch(batch)
+    assert seen[-1] == described(entry)
