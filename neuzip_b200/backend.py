@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import enum
 import functools
+import math
 import threading
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence
@@ -389,13 +390,15 @@ class CodecBackend:
         return out
 
     def read_shaped(self, name: str, shape) -> torch.Tensor:
-        """`read` into a tensor of the given shape (as many elements as were written)."""
+        """`read` into a tensor of the given shape, as ``read(name).view(*shape)`` gives it (one
+        size may be -1; a shape that does not fit raises the same error)."""
         entry = self._get(name)
         if entry is None:
             raise RuntimeError("Data not found")
-        out = torch.empty(shape, dtype=torch.bfloat16, device=_CUDA)
-        if out.numel() != entry.numel:
-            raise RuntimeError(f"shape '{list(shape)}' is invalid for input of size {entry.numel}")
+        if math.prod(shape) == entry.numel:
+            out = torch.empty(shape, dtype=torch.bfloat16, device=_CUDA)
+        else:
+            out = torch.empty(entry.numel, dtype=torch.bfloat16, device=_CUDA).view(tuple(shape))
         self._decode(entry, out)
         return out
 
