@@ -386,10 +386,7 @@ linear_kernel(const LinearArgs p, const __grid_constant__ CUtensorMap x_map) {
   const bool is_dec = warp < (uint32_t)kLinDecWarps;
   const bool is_mma = warp == (uint32_t)kLinDecWarps;
 
-  // a dependent launch (the kernel that adds up the column segments) may be set up now; it
-  // waits for this grid to complete before it reads anything
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  // ---- barriers and tensor memory
+  // ---- barriers
   if (threadIdx.x == 0) *abort_flag = 0;
   if (is_dec) {
     if (lane == 0) mbar_init(misc_a + kBarWarp + 8 * warp, 1);
@@ -402,12 +399,6 @@ linear_kernel(const LinearArgs p, const __grid_constant__ CUtensorMap x_map) {
       }
       mbar_init(misc_a + kBarDone, 1);
     }
-    __syncwarp();
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     misc_a + kTmemSlot),
-                 "r"(p.tmem_cols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (lane == 0) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -416,9 +407,20 @@ linear_kernel(const LinearArgs p, const __grid_constant__ CUtensorMap x_map) {
   __syncwarp();
 
   // The launch may overlap the tail of the kernel before it (programmatic stream
-  // serialisation): barriers, flags and tensor memory are set up by now, global memory is not
-  // touched before that kernel has completed.
+  // serialisation): barriers and flags are set up by now, global memory is not touched before
+  // that kernel has completed.
   asm volatile("griddepcontrol.wait;" ::: "memory");
+
+  // ---- tensor memory.  The allocation blocks until columns are free on this SM, so it comes
+  // after the wait: a CTA that held columns while it waited for the kernel before could keep
+  // that kernel's last CTAs from theirs, and neither would ever go on.
+  if (is_mma) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     misc_a + kTmemSlot),
+                 "r"(p.tmem_cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
 
   // ---- plan and stage this warp's two units, build the decode table meanwhile
   const Header *h = reinterpret_cast<const Header *>(a.container);
@@ -443,6 +445,10 @@ linear_kernel(const LinearArgs p, const __grid_constant__ CUtensorMap x_map) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  // This CTA has its tensor memory: a dependent launch (the kernel that adds up the column
+  // segments, or the next call's) may be set up now; it waits for this grid to complete before
+  // it reads or allocates anything.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   uint32_t pb;
   const uint32_t bad = table_verdict(cum_sh, flag_sh, pb);
   const uint32_t tmem = *tmem_slot;
