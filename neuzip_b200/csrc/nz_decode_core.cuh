@@ -12,10 +12,12 @@
 
 namespace nz {
 
-// A wait is a bounded number of tries; each may suspend the thread for kWaitHintNs, so that
-// a warp that waits takes no issue slots from those that decode.
+// A wait is a bounded number of tries; each may suspend the thread for up to kWaitHintNs, so
+// that a warp that waits takes no issue slots from those that decode.  The hint is an upper
+// limit only, a try may return at once: the number of tries is what a slow copy (a container in
+// host memory) has to get by with, about a second at the most.
 constexpr uint32_t kWaitHintNs = 1000;
-constexpr uint32_t kMaxWaitIters = 1u << 16;
+constexpr uint32_t kMaxWaitIters = 1u << 20;
 
 // ------------------------------------------------------------- PTX helpers
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {

@@ -20,3 +20,11 @@ def test_tensor_memory_is_taken_between_the_wait_and_the_trigger():
     barrier = body.index("__syncthreads()", alloc)
     assert body.count("griddepcontrol.wait") == body.count("tcgen05.alloc") == 1
     assert wait < alloc < barrier < body.index("griddepcontrol.launch_dependents")
+
+
+def test_waits_give_a_slow_copy_a_million_tries():
+    text = source("nz_decode_core.cuh")
+    tries = re.search(r"kMaxWaitIters = 1u << (\d+);", text)
+    hint = re.search(r"kWaitHintNs = (\d+);", text)
+    assert int(tries.group(1)) >= 20                               # how early a try returns is open
+    assert int(hint.group(1)) << int(tries.group(1)) <= 2 << 30    # and the wait stays bounded
