@@ -312,10 +312,10 @@ class CodecBackend:
         Header slots (one pinned buffer, 64 bytes each) and events are pooled: a write
         allocates no pinned memory and creates no event once the pools are warm."""
         with self._pending_lock:
-            if replaced is not None:
+            if replaced is not None and replaced.pending is not None:
                 # overwritten before it was ever settled: its slot and event go back (a copy
                 # still in flight into the slot lands before the next one, same stream)
-                self._release_pending(replaced)
+                self._give_back(replaced)
             if not self._hdr_free:
                 self._grow_header_pool()
             slot = self._hdr_free.pop()
@@ -336,13 +336,16 @@ class CodecBackend:
         self._hdr_free.extend(range(256 * index + 255, 256 * index - 1, -1))
 
     def _release_pending(self, entry: _Entry) -> None:
-        """Slot and event of an entry that will not be settled (any more) go back, once."""
+        """For an entry that will not be settled any more."""
         with self._pending_lock:
             if entry.pending is not None:
-                slot, event = entry.pending
-                entry.pending = None
-                self._hdr_free.append(slot)
-                self._event_pool.append(event)
+                self._give_back(entry)
+
+    def _give_back(self, entry: _Entry) -> None:
+        slot, event = entry.pending
+        entry.pending = None
+        self._hdr_free.append(slot)
+        self._event_pool.append(event)
 
     def _settle(self, entry: _Entry, block: bool) -> None:
         pending = entry.pending
@@ -359,7 +362,7 @@ class CodecBackend:
             total, words = ctypes.c_uint64(0), ctypes.c_uint32(0)
             rc = self._lib.nz_parse_header(self._hdr_base[slot >> 8] + 64 * (slot & 255),
                                            ctypes.byref(total), ctypes.byref(words))
-            self._release_pending(entry)
+            self._give_back(entry)
             if rc:
                 raise _lib.NeuzipError("write produced no NZR1 container")
             # a reader that sees the new container also sees its largest unit
