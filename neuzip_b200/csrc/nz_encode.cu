@@ -875,23 +875,42 @@ __device__ __forceinline__ uint32_t encode_update(uint32_t x, const uint4 e, uin
   return q * cm + (x + e.w);
 }
 
-// One step, the word going to shared memory: `pos` is the shared address of the lane's next
-// free 16-bit place and counts down.
-template <bool BIG>
-__device__ __forceinline__ void encode_step_sh(uint32_t &x, uint32_t &pos, const uint4 e,
-                                               uint32_t pow_m) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ge.u32 p, %0, %2;\n\t"
-      "@p st.shared.u16 [%1], %0;\n\t"
-      "@p shr.u32 %0, %0, 16;\n\t"
-      "@p add.u32 %1, %1, -2;\n\t"
-      "}"
-      : "+r"(x), "+r"(pos)
-      : "r"(e.y));
-  x = encode_update<BIG>(x, e, pow_m);
-}
+// Where a lane's words go, last word first.
+// SliceSink: down its slice of the warp's cell in shared memory; `pos` is the shared address of
+// the next free 16-bit place.  A lane whose slice could run out inside a block (`limit`) starts
+// over at its top and counts what it has emitted in `spilled`: the unit is coded a second time.
+struct SliceSink {
+  uint32_t pos, top, limit, spilled;
+  __device__ __forceinline__ void block() {
+    if (pos < limit) {
+      spilled += (top - pos) >> 1;
+      pos = top;
+    }
+  }
+  __device__ __forceinline__ void renormalise(uint32_t &x, uint32_t bound) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "setp.ge.u32 p, %0, %2;\n\t"
+        "@p st.shared.u16 [%1], %0;\n\t"
+        "@p shr.u32 %0, %0, 16;\n\t"
+        "@p add.u32 %1, %1, -2;\n\t"
+        "}"
+        : "+r"(x), "+r"(pos)
+        : "r"(bound));
+  }
+};
+// SlotSink: to their final places in the unit's slot (the second coding knows them).
+struct SlotSink {
+  uint16_t *at;              // one past the next place
+  __device__ __forceinline__ void block() {}
+  __device__ __forceinline__ void renormalise(uint32_t &x, uint32_t bound) {
+    if (x >= bound) {
+      *--at = (uint16_t)x;
+      x >>= 16;
+    }
+  }
+};
 
 // The S+1 bytes of packed fields of 8 elements, in memory order (f0: first four bytes, f1: the
 // rest at precision 7), from their words and rounded magnitudes.
@@ -925,49 +944,15 @@ __device__ __forceinline__ void pack_fields(const uint32_t (&w)[4], const uint32
   }
 }
 
-// Second coding of a unit whose words did not fit the shared-memory slices: the
-// lengths are known from the first attempt, so every word goes straight to its
-// final place in the slot (global memory).
-template <int S>
-__device__ __noinline__ void encode_unit_in_place(const uint16_t *__restrict__ in, uint64_t n,
-                                                  uint32_t LS, uint32_t cols, uint64_t first,
-                                                  uint32_t pad, const uint4 *tab, uint32_t pow_m,
-                                                  uint16_t *slot, uint32_t offset, uint32_t words,
-                                                  uint32_t padded, uint32_t lane) {
-  // the lane's stream occupies slot[offset .. offset + padded); words are emitted
-  // backwards from offset + words - 1, the state ends up in the first two places
-  uint16_t *mine = slot + offset;
-  uint32_t at = words;
-  uint32_t x = kStateLow;
-  for (int32_t blk = (int32_t)(LS / 8) - 1; blk >= 0; --blk) {
-    uint32_t lo, hi;
-    load_group<S>(in, first + (uint64_t)blk * 256 + lane * 8, n, cols, pad, nullptr, false, lo, hi);
-#pragma unroll 1
-    for (int t = 7; t >= 0; --t) {
-      const uint4 e = tab[((t < 4 ? lo : hi) >> (8 * (t & 3))) & 0xFFu];
-      if (x >= e.y) {
-        mine[--at] = (uint16_t)x;
-        x >>= 16;
-      }
-      x = encode_update<true>(x, e, pow_m);
-    }
-  }
-  mine[0] = (uint16_t)(x & 0xFFFFu);
-  mine[1] = (uint16_t)(x >> 16);
-  for (uint32_t k = words; k < padded; ++k) mine[k] = 0;
-}
-
-// The whole blocks of one unit, last to first.  Software pipeline: the 16 bytes of block
-// b - 2 are requested while block b is coded; the table entries are fetched two symbols ahead
-// (they depend on the symbols only), so neither latency sits on the chain state -> state.
-// A lane whose slice could run out inside a block (`limit`) starts over at its top and counts
-// what it has emitted in `spilled`: the unit is then coded a second time.
-template <int S, bool BIG>
+// The first n_blocks blocks of one unit, whole ones, last to first.  Software pipeline: the 16
+// bytes of block b - 2 are requested while block b is coded; the table entries are fetched two
+// symbols ahead (they depend on the symbols only), so neither latency sits on the chain state ->
+// state.
+template <int S, bool BIG, bool STORE, class Sink>
 __device__ __forceinline__ void encode_blocks(const uint16_t *__restrict__ src, uint32_t step,
                                               uint8_t *__restrict__ fdst, uint32_t n_blocks,
-                                              const uint4 *tab, uint32_t pow_m, uint32_t top,
-                                              uint32_t limit, uint32_t &x, uint32_t &pos,
-                                              uint32_t &spilled) {
+                                              const uint4 *tab, uint32_t pow_m, uint32_t &x,
+                                              Sink &sink) {
   uint4 cur = __ldg(reinterpret_cast<const uint4 *>(src)), nxt = cur;
   src -= step;
   if (n_blocks > 1) nxt = __ldg(reinterpret_cast<const uint4 *>(src));
@@ -986,21 +971,80 @@ __device__ __forceinline__ void encode_blocks(const uint16_t *__restrict__ src, 
     cur = nxt;
     src -= step;
     if (b > 2) nxt = __ldg(reinterpret_cast<const uint4 *>(src));
-    pack_fields<S>(w, k, f0, f1);
-    store_fields<S>(fdst, f0, f1);
-    fdst -= 32 * (S + 1);
-    if (pos < limit) {
-      spilled += (top - pos) >> 1;
-      pos = top;
+    if (STORE) {
+      pack_fields<S>(w, k, f0, f1);
+      store_fields<S>(fdst, f0, f1);
+      fdst -= 32 * (S + 1);
     }
+    sink.block();
 #pragma unroll
     for (int t = 7; t >= 0; --t) {
       const uint4 e = e0;
       e0 = e1;
       if (t >= 2) e1 = entry(t - 2);
-      encode_step_sh<BIG>(x, pos, e, pow_m);
+      sink.renormalise(x, e.y);
+      x = encode_update<BIG>(x, e, pow_m);
     }
   }
+}
+
+// What lies behind the `count / 256` whole blocks of a ragged unit, last to first: blocks of
+// nothing but the pad symbol (no loads), then the block that ends the tensor.  The whole blocks
+// take encode_blocks: a small tensor lasts as long as its ragged unit (1551 x 1134 elements at
+// precision 1: 69 us with all of its blocks loaded and coded one by one here, 49 like this).
+template <int S, class Sink>
+__device__ __forceinline__ void encode_tail(const uint16_t *__restrict__ in, uint64_t n, uint32_t first,
+                                            uint32_t count, uint32_t n_blocks, uint32_t cols,
+                                            uint32_t pad, uint8_t *frac_out, bool store,
+                                            const uint4 *tab, uint32_t pow_m, uint32_t lane,
+                                            uint32_t &x, Sink &sink) {
+  const uint4 e = tab[pad];
+  const uint32_t with_elements = (count + 255) >> 8;
+#pragma unroll 1
+  for (uint32_t b = n_blocks; b > with_elements; --b) {
+    sink.block();
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      sink.renormalise(x, e.y);
+      x = encode_update<true>(x, e, pow_m);
+    }
+  }
+  if (count & 255) {
+    uint32_t lo, hi;
+    load_group<S>(in, (uint64_t)first + (uint64_t)(with_elements - 1) * 256 + lane * 8, n, cols, pad,
+                  frac_out, store, lo, hi);
+    sink.block();
+#pragma unroll 1
+    for (int t = 7; t >= 0; --t) {
+      const uint4 f = tab[((t < 4 ? lo : hi) >> (8 * (t & 3))) & 0xFFu];
+      sink.renormalise(x, f.y);
+      x = encode_update<true>(x, f, pow_m);
+    }
+  }
+}
+
+// Second coding of a unit whose words did not fit the shared-memory slices: the
+// lengths are known from the first attempt, so every word goes straight to its
+// final place in the slot (global memory).
+template <int S>
+__device__ __noinline__ void encode_unit_in_place(const uint16_t *__restrict__ in, uint64_t n,
+                                                  uint32_t n_blocks, uint32_t cols, uint32_t first,
+                                                  uint32_t count, uint32_t pad, const uint4 *tab,
+                                                  uint32_t pow_m, uint16_t *slot, uint32_t offset,
+                                                  uint32_t words, uint32_t padded, uint32_t lane) {
+  // the lane's stream occupies slot[offset .. offset + padded); words are emitted
+  // backwards from offset + words - 1, the state ends up in the first two places
+  uint16_t *mine = slot + offset;
+  SlotSink sink = {mine + words};
+  uint32_t x = kStateLow;
+  if ((count >> 8) < n_blocks)
+    encode_tail<S>(in, n, first, count, n_blocks, cols, pad, nullptr, false, tab, pow_m, lane, x, sink);
+  if (count >> 8)
+    encode_blocks<S, true, false>(in + source_index32(first + ((count >> 8) - 1) * 256 + lane * 8, cols),
+                                  cols ? 64u : 256u, nullptr, count >> 8, tab, pow_m, x, sink);
+  mine[0] = (uint16_t)(x & 0xFFFFu);
+  mine[1] = (uint16_t)(x >> 16);
+  for (uint32_t k = words; k < padded; ++k) mine[k] = 0;
 }
 
 // What bounds it: the integer pipes (about 13 instructions per symbol, one of them a high
@@ -1047,34 +1091,22 @@ bf16_encode_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uin
     if (u + gridDim.x * n_warps >= n_units) dependent_trigger();
     const uint32_t first = u * U;                      // element indices are below 2^32
     const uint32_t left = (uint32_t)n - first, count = left < U ? left : U;
-    uint32_t x = kStateLow, pos = top, spilled = 0;
-    if (count == U) {
-      // whole units walk two pointers down, block by block (in operand order a unit's blocks
-      // are 64 elements apart in the lane's row; otherwise 256)
-      const uint32_t e_last = first + (n_blocks - 1) * 256 + lane * 8;
+    uint32_t x = kStateLow;
+    SliceSink sink = {top, top, limit, 0};
+    // whole blocks walk two pointers down (in operand order a unit's blocks are 64 elements
+    // apart in the lane's row; otherwise 256); the tensor's last unit can have a ragged tail
+    const uint32_t whole = count >> 8;
+    if (whole < n_blocks)
+      encode_tail<S>(in, n, first, count, n_blocks, cols, pad, frac_out, true, tab, pow_m, lane, x, sink);
+    if (whole) {
+      const uint32_t e_last = first + (whole - 1) * 256 + lane * 8;
       const uint16_t *src = in + source_index32(e_last, cols);
       uint8_t *fdst = frac_out + ((uint64_t)e_last * (S + 1) >> 3);
       const uint32_t step = cols ? 64u : 256u;
-      if (big)
-        encode_blocks<S, true>(src, step, fdst, n_blocks, tab, pow_m, top, limit, x, pos, spilled);
-      else
-        encode_blocks<S, false>(src, step, fdst, n_blocks, tab, pow_m, top, limit, x, pos, spilled);
-    } else {
-      // the tensor's last unit can be ragged and takes the guarded loads
-#pragma unroll 1
-      for (int32_t blk = (int32_t)n_blocks - 1; blk >= 0; --blk) {
-        uint32_t lo, hi;
-        load_group<S>(in, (uint64_t)first + (uint64_t)blk * 256 + lane * 8, n, cols, pad, frac_out, true,
-                      lo, hi);
-        if (pos < limit) {
-          spilled += (top - pos) >> 1;
-          pos = top;
-        }
-#pragma unroll 1
-        for (int t = 7; t >= 0; --t)
-          encode_step_sh<true>(x, pos, tab[((t < 4 ? lo : hi) >> (8 * (t & 3))) & 0xFFu], pow_m);
-      }
+      if (big) encode_blocks<S, true, true>(src, step, fdst, whole, tab, pow_m, x, sink);
+      else encode_blocks<S, false, true>(src, step, fdst, whole, tab, pow_m, x, sink);
     }
+    const uint32_t pos = sink.pos, spilled = sink.spilled;
     const uint32_t words = spilled + ((top - pos) >> 1) + 2;
     const uint32_t q = (words + lenq - 1) / lenq;
     const uint32_t padded = q * lenq;
@@ -1101,8 +1133,8 @@ bf16_encode_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uin
     if (__any_sync(0xFFFFFFFFu, spilled != 0)) {
       // did not fit the slices: code it again, straight into the slot
       reinterpret_cast<uint8_t *>(slot)[lane] = (uint8_t)q;
-      encode_unit_in_place<S>(in, n, LS, cols, first, pad, tab, pow_m, slot, 16 + incl - padded, words,
-                              padded, lane);
+      encode_unit_in_place<S>(in, n, n_blocks, cols, first, count, pad, tab, pow_m, slot,
+                              16 + incl - padded, words, padded, lane);
       continue;
     }
     // state in front of the emitted words, then the 32 streams back to back

@@ -1,7 +1,8 @@
 """Branches of the fused encoder, each against the oracle byte for byte: a symbol with more
 than half of the slots (the remainder is checked), units above 3 bits per symbol (squeezed in
 place), lanes that outgrow their slice (the unit is coded a second time), length quanta of two
-words, ragged last units, and tensors whose units do not fill the GPU evenly."""
+words, ragged last units (whole blocks, the block that ends the tensor, blocks of
+nothing but padding), and tensors whose units do not fill the GPU evenly."""
 import numpy as np
 import pytest
 import torch
@@ -21,6 +22,8 @@ def bits_of(kind, n, seed):
         exp = np.full(n, 121)
     elif kind == "uniform10":                      # 3.3 bits per symbol
         exp = rng.integers(115, 125, n)
+    elif kind == "raw":                            # runs of 2048 that do not compress, among others
+        exp = np.where(np.arange(n) // 2048 % 3 == 1, rng.integers(1, 255, n), rng.integers(118, 122, n))
     elif kind == "uniform60":                      # 5.9 bits: every lane outgrows its slice
         exp = rng.integers(80, 140, n)
     else:                                          # one lane of 32 has the rare exponents
@@ -40,6 +43,26 @@ def test_encoder_branches(s, kind):
             c_ref, f_ref = O.compress_bf16(bits, s, S)
             assert np.array_equal(cont.cpu().numpy(), c_ref), (s, kind, S, n)
             assert np.array_equal(frac.cpu().numpy(), f_ref), (s, kind, S, n)
+
+
+def check(bits, s, S):
+    cont, frac, _ = A.compress(A.from_bits(bits), s, S)
+    c_ref, f_ref = O.compress_bf16(bits, s, S)
+    assert np.array_equal(cont.cpu().numpy(), c_ref), (s, S, bits.size)
+    assert np.array_equal(frac.cpu().numpy(), f_ref), (s, S, bits.size)
+    return c_ref
+
+
+@pytest.mark.parametrize("s", (7, 3, 1, 0))
+@pytest.mark.parametrize("kind", ("peaked", "uniform10", "uniform60", "raw"))
+def test_ragged_last_units(s, kind):
+    # the last unit's count around every edge of its three parts, alone and behind whole units
+    for S in (8, 64, 384):
+        U = 32 * S
+        for count in {1, 7, 8, 255, 256, 257, 511, 512, U // 2 + 3, U - 257, U - 256, U - 255, U - 1}:
+            for units in (0, 3):
+                if 0 < count < U:
+                    check(bits_of(kind, units * U + count, S + count), s, S)
 
 
 @pytest.mark.parametrize("units", (255, 256, 257, 148 * 48 * 3 + 4, 255 * 512 + 1))
