@@ -1250,11 +1250,33 @@ place_units_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uin
     const uint32_t size = __shfl_sync(0xFFFFFFFFu, mine, j), w0 = __shfl_sync(0xFFFFFFFFu, start, j);
     uint16_t *dst = payload + w0;
     if (size & kRawFlag) {
-      const uint64_t first = (uint64_t)u * U;
-      const uint64_t count = (n - first < U) ? (n - first) : U;
+      const uint32_t first = u * (uint32_t)U;                 // element indices are below 2^32
+      const uint32_t left = (uint32_t)n - first, count = left < (uint32_t)U ? left : (uint32_t)U;
+      // 8 elements of a lane are one 16-byte load and, as the unit starts on any 16-bit word of
+      // the payload, four 16-bit stores; two loads of a lane are in flight.  (One by one, behind a
+      // division each: 179 us for 11008 x 4096 elements with raw rows instead of 131.)
+      constexpr uint32_t kRawBatch = 2;
+      const uint32_t groups = count >> 3;
+      for (uint32_t g0 = lane; g0 < groups; g0 += 32 * kRawBatch) {
+        uint4 q[kRawBatch];
+#pragma unroll
+        for (uint32_t i = 0; i < kRawBatch; ++i)
+          if (g0 + 32 * i < groups)
+            q[i] = __ldg(reinterpret_cast<const uint4 *>(in + source_index32(first + (g0 + 32 * i) * 8, cols)));
+#pragma unroll
+        for (uint32_t i = 0; i < kRawBatch; ++i) {
+          if (g0 + 32 * i >= groups) break;
+          const uint32_t w[4] = {q[i].x, q[i].y, q[i].z, q[i].w};
+#pragma unroll
+          for (uint32_t j = 0; j < 4; ++j) {
+            const uint32_t r = round_pair<S>(w[j]);           // exponents in bits 7-14 and 23-30
+            dst[(g0 + 32 * i) * 4 + j] = (uint16_t)(((r >> 7) & 0xFFu) | ((r >> 15) & 0xFF00u));
+          }
+        }
+      }
       uint8_t *d8 = reinterpret_cast<uint8_t *>(dst);
-      for (uint64_t i = lane; i < count; i += 32)
-        d8[i] = (uint8_t)exp_of<S>(in[source_index(first + i, cols)]);
+      const uint32_t e = groups * 8 + lane;                   // fewer than 8 are left
+      if (e < count) d8[e] = (uint8_t)exp_of<S>(in[source_index32(first + e, cols)]);
       if ((count & 1) && lane == 0) d8[count] = 0;
       continue;
     }

@@ -1,7 +1,7 @@
 """Branches of the fused encoder, each against the oracle byte for byte: a symbol with more
 than half of the slots (the remainder is checked), units above 3 bits per symbol (squeezed in
-place), lanes that outgrow their slice (the unit is coded a second time), length quanta of two
-words, ragged last units (whole blocks, the block that ends the tensor, blocks of
+place), lanes that outgrow their slice (the unit is coded a second time), units stored raw, length
+quanta of two words, ragged last units (whole blocks, the block that ends the tensor, blocks of
 nothing but padding), and tensors whose units do not fill the GPU evenly."""
 import numpy as np
 import pytest
@@ -63,6 +63,26 @@ def test_ragged_last_units(s, kind):
             for units in (0, 3):
                 if 0 < count < U:
                     check(bits_of(kind, units * U + count, S + count), s, S)
+
+
+@pytest.mark.parametrize("s", (7, 3, 1, 0))
+def test_raw_units(s):
+    for S in (8, 64):
+        for n in (2048 * 9, 2048 * 4 + 1, 2048 * 4 + 7, 2048 * 4 + 2043):
+            cont = check(bits_of("raw", n, S + n), s, S)
+            units = -(-n // (32 * S))
+            offs = np.frombuffer(cont.tobytes(), dtype=np.uint32, count=units, offset=576)
+            assert (offs >> 31).any() and not (offs >> 31).all()
+
+
+@pytest.mark.parametrize("s", (7, 1))
+def test_raw_units_in_operand_order(s):
+    rows, cols, S = 64, 512, 64
+    bits = bits_of("raw", rows * cols, 5)
+    cont, frac, _ = A.compress_operand(A.from_bits(bits), rows, cols, s, S)
+    c_ref, f_ref = O.compress_bf16(O.to_operand_order(bits, rows, cols), s, S)
+    assert np.array_equal(cont.cpu().numpy(), c_ref) and np.array_equal(frac.cpu().numpy(), f_ref)
+    assert (np.frombuffer(c_ref.tobytes(), dtype=np.uint32, count=16, offset=576) >> 31).any()
 
 
 @pytest.mark.parametrize("units", (255, 256, 257, 148 * 48 * 3 + 4, 255 * 512 + 1))
