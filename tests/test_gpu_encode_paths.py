@@ -85,6 +85,17 @@ def test_raw_units_in_operand_order(s):
     assert (np.frombuffer(c_ref.tobytes(), dtype=np.uint32, count=16, offset=576) >> 31).any()
 
 
+@pytest.mark.parametrize("units", (147, 148, 149, 148 * 8, 148 * 8 + 1, 148 * 9, 148 * 16 + 1, 148 * 33))
+def test_split_over_the_sms(units):
+    # a unit per warp on every SM, several blocks per SM, and more units than warps
+    check(bits_of("peaked", 256 * units - 5, 11), 7, 8)
+
+
+@pytest.mark.parametrize("S", (512, 640, 768, 1024))
+def test_long_units_beyond_one_wave(S):
+    check(bits_of("uniform10", 32 * S * (148 * 8 + 3) - 77, 12), 1, S)
+
+
 @pytest.mark.parametrize("units", (255, 256, 257, 148 * 48 * 3 + 4, 255 * 512 + 1))
 def test_many_units(units):
     # chunks of one and more units, several units per warp, and offsets from the scan kernel
