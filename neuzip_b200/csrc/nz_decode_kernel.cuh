@@ -609,6 +609,59 @@ __device__ __forceinline__ void decode_rest(const DecodeArgs &a, LaneState &st, 
   }
 }
 
+// A raw unit: its exponent bytes are stored as they are, from any 16-bit word of the payload on.
+// Block by block like a coded unit, bytes and fractions fetched a block ahead; what is left of
+// a ragged one element by element.  (All of it element by element: 282 us for 11008 x 4096
+// elements with raw rows; units next to one another, as those of a row are, meet in one warp.)
+// A function of its own, given what it needs one by one, so that the registers and the code of
+// the loops above stay as they are.  `e` is the unit's first element in the tensor, `out` where
+// the lane's first element goes (bf16, or bytes without MERGE), `adv` the distance between its
+// blocks.
+template <int S, bool MERGE>
+__device__ __noinline__ void emit_raw_unit(const uint8_t *src, const uint8_t *frac, void *out, uint32_t e,
+                                           uint32_t count, uint32_t adv, bool canon,
+                                           const uint8_t *norm, uint32_t norm_lg) {
+  constexpr uint32_t kFracStride = 32u * (S + 1);
+  const uint32_t lane = threadIdx.x & 31, full_blocks = count >> 8;
+  uint16_t *out_lane = reinterpret_cast<uint16_t *>(out);
+  uint8_t *exp_lane = reinterpret_cast<uint8_t *>(out);
+  const uint16_t *raw = reinterpret_cast<const uint16_t *>(src) + lane * 4;
+  const uint8_t *frac_lane = MERGE ? frac + ((uint64_t)(e + lane * 8) * (S + 1) >> 3) : nullptr;
+  uint32_t lo = 0, hi = 0;
+  uint64_t bits = 0;
+  auto fetch = [&]() {
+    lo = __ldg(raw) | ((uint32_t)__ldg(raw + 1) << 16);
+    hi = __ldg(raw + 2) | ((uint32_t)__ldg(raw + 3) << 16);
+    raw += 128;
+    if (MERGE) {
+      bits = load_frac<S>(frac_lane);
+      frac_lane += kFracStride;
+    }
+  };
+  if (full_blocks) fetch();
+#pragma unroll 1
+  for (uint32_t b = 0; b < full_blocks; ++b) {
+    const uint32_t sym[2] = {lo, hi};
+    const uint64_t now = bits;
+    if (b + 1 < full_blocks) fetch();
+    if (MERGE) {
+      uint32_t w[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const uint32_t pair = sym[t >> 1] >> (16 * (t & 1));
+        w[t] = merge_word<S>((pair & 0xFFu) << kEntSymShift, (pair << (kEntSymShift - 8)) & 0x7F800000u, now, t);
+        if (canon) w[t] = canon_word(w[t]);
+      }
+      if (norm) norm_words(w, norm_bytes(norm, norm_lg, e + lane * 8 + b * 256), norm_lg);
+      __stcs(reinterpret_cast<uint4 *>(out_lane), make_uint4(w[0], w[1], w[2], w[3]));
+      out_lane += adv;
+    } else {
+      __stcs(reinterpret_cast<uint2 *>(exp_lane), make_uint2(sym[0], sym[1]));
+      exp_lane += 256;
+    }
+  }
+}
+
 // Decode one unit on its own (raw units, odd counts).
 template <int S, bool MERGE>
 __device__ __forceinline__ void decode_single(const DecodeArgs &a, const UnitPlan &pl, uint32_t u,
@@ -616,11 +669,15 @@ __device__ __forceinline__ void decode_single(const DecodeArgs &a, const UnitPla
                                               const uint8_t *payload, uint32_t lenq,
                                               uint32_t lane) {
   if (pl.kind == kUnitRaw) {
-    const uint64_t U = 32ull * a.S;
-    const uint64_t first = (uint64_t)u * U;
-    const uint64_t count = (a.n - first < U) ? (a.n - first) : U;
+    const uint32_t U = 32u * a.S, first = u * U;
+    const uint32_t count = u < a.full_units ? U : (uint32_t)a.n - first;
     const uint8_t *src = payload + pl.byte0();
-    for (uint64_t i = lane; i < count; i += 32) emit_guarded<S, MERGE>(src[i], first + i, delta, a);
+    const int64_t o = (int64_t)unit_out_index(a, u, lane) + delta;      // (exponents: stream order)
+    emit_raw_unit<S, MERGE>(src, a.frac, MERGE ? (void *)(a.out_bf16 + o) : (void *)(a.out_exp + o), first,
+                            count, a.tile_cols ? 64u : 256u, a.canon != 0, a.norm, a.norm_lg);
+#pragma unroll 1
+    for (uint32_t i = (count & ~255u) + lane; i < count; i += 32)
+      emit_guarded<S, MERGE>(src[i], (uint64_t)first + i, delta, a);
     return;
   }
   if (pl.kind != kUnitCoded) return;
