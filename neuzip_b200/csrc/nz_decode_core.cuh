@@ -120,9 +120,9 @@ __device__ __forceinline__ uint32_t entry_symbol(uint32_t ent) { return ent >> k
 // ROW == 0: the table is wide; returns the wide entry.  The state update is
 // f*(q - 4096) + (f*4096 + offset) = f*q + offset (mod 2^32), so that the entry's low 23
 // bits serve as the addend unshifted.
-// ROW == kAnyRow: either table, looked up for every symbol (units decoded on their own);
-// returns an entry with the symbol where the wide layout has it.
-constexpr int kAnyRow = -1;
+// ROW == kNarrowRow: the table is narrow, its size is looked up (units decoded on their own);
+// returns the entry with the symbol where the wide layout has it.
+constexpr int kNarrowRow = -1;
 template <int ROW, int PB = 0>
 __device__ __forceinline__ uint32_t decode_step(LaneState &st, const LutView &lv) {
   uint32_t ent;
@@ -145,7 +145,7 @@ __device__ __forceinline__ uint32_t decode_step(LaneState &st, const LutView &lv
         "}"
         : "=&r"(ent), "+r"(st.x), "+r"(st.p), "+r"(st.w)
         : "r"(lv.base), "r"(lv.k64k), "n"((1 << PB) - 1), "n"(PB), "n"(1 << ROW));
-  } else if (ROW == kAnyRow && lv.narrow) {
+  } else if constexpr (ROW == kNarrowRow) {
     asm volatile(
         "{\n\t"
         ".reg .b32 a, q, f, b;\n\t"
@@ -187,6 +187,10 @@ __device__ __forceinline__ uint32_t decode_step(LaneState &st, const LutView &lv
         : "r"(lv.base), "r"(lv.mask), "r"(lv.stride), "r"(lv.pb), "r"(lv.k64k));
   }
   return ent;
+}
+// One symbol of either table, for code that runs too rarely to have a loop for each.
+__device__ __forceinline__ uint32_t decode_step_any(LaneState &st, const LutView &lv) {
+  return lv.narrow ? decode_step<kNarrowRow>(st, lv) : decode_step<0>(st, lv);
 }
 // Byte selector that joins the symbols of two entries (see the layouts above): from narrow
 // entries when ROW > 0, from entries in the wide layout when ROW == 0.

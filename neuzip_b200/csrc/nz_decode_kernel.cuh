@@ -131,10 +131,11 @@ __device__ __forceinline__ void norm_words(uint32_t (&w)[4], uint64_t bytes, uin
   }
 }
 
-// Decode blocks b0 .. n_blocks - 1 of one unit for this lane, whatever the table's layout
-// (units decoded on their own: few of them, so the code is kept small).  `e` is the lane's
-// first element of the unit.  The packed fractions are fetched a block ahead of their use.
-template <int S, bool MERGE>
+// Decode blocks b0 .. n_blocks - 1 of one unit for this lane (units decoded on their own).  ROW
+// is kNarrowRow or 0, by the table's layout: looked up once per unit and not per symbol, which
+// costs a sixth of the rate.  `e` is the lane's first element of the unit.  The packed fractions
+// are fetched a block ahead of their use.
+template <int S, bool MERGE, int ROW>
 __device__ __forceinline__ void decode_blocks(const DecodeArgs &a, LaneState &st, const LutView &lut,
                                               uint32_t b0, uint32_t n_blocks, uint32_t e,
                                               uint16_t *out_lane, uint8_t *exp_lane, uint32_t adv,
@@ -151,7 +152,7 @@ __device__ __forceinline__ void decode_blocks(const DecodeArgs &a, LaneState &st
     const uint64_t scales = MERGE && a.norm ? norm_bytes(a.norm, a.norm_lg, e + b * 256) : 0;
     uint32_t ent[8];
 #pragma unroll
-    for (int t = 0; t < 8; ++t) ent[t] = decode_step<kAnyRow>(st, lut);
+    for (int t = 0; t < 8; ++t) ent[t] = decode_step<ROW>(st, lut);
     if (MERGE) {
       uint32_t w[4];
 #pragma unroll
@@ -356,14 +357,10 @@ struct UpdateSinkT {
 // Start the copies of a group's first packed fractions into the warp's ring.  They depend on
 // nothing that is decoded, so the caller issues them before it waits for the coded units:
 // the two latencies overlap.  `ring` carries the lane's offset in a block (8 or 4 bytes).
-// s = 0 and 1: block counts that are a multiple of four go through the grouped ring
-__device__ __forceinline__ bool ring_by_group(int s, uint32_t n_blocks) {
-  return (s == 0 || s == 1) && (n_blocks & 3) == 0;
-}
 template <int S, int C>
 __device__ __forceinline__ void group_async(uint32_t ring, const uint8_t *(&frac)[kChains],
                                             uint32_t g) {
-  // four blocks of a unit are 128 (s=0) or 256 (s=1) contiguous bytes, copied by the whole
+  // s = 0 and 1: four blocks of a unit are 128 or 256 contiguous bytes, copied by the whole
   // warp (4 or 8 bytes per lane)
   constexpr uint32_t kLaneBytes = 4u * (S + 1);          // per lane and group
   constexpr uint32_t kGroupBytes = 32u * kLaneBytes;     // per unit and group
@@ -398,7 +395,7 @@ __device__ __forceinline__ void ring_prologue(uint32_t ring, const uint8_t *(&fr
       }
       frac_commit();
     }
-  } else if (ring_by_group(S, n_blocks)) {
+  } else if (n_blocks >= 4) {
     group_async<S, C>(ring, frac, 0);
   }
 }
@@ -411,19 +408,22 @@ __device__ __forceinline__ void ring_prologue(uint32_t ring, const uint8_t *(&fr
 // are fetched four blocks at a time by the whole warp.  The caller has started the
 // first copies (ring_prologue); returns true when the next group's first copies are under
 // way in their place.
-template <int S, bool MERGE, int ROW, int C, typename Sink>
+//
+// CANON: the tensor has NaN to rewrite (tables in the wide layout only); a template parameter,
+// because the test at run time costs a fifth of the loop's rate (116 instead of 98 cycles a step
+// in a lone warp).
+template <int S, bool MERGE, int ROW, bool CANON, int C, typename Sink>
 __device__ __forceinline__ bool decode_blocks_multi(LaneState (&st)[kChains], const LutView &lut,
-                                                    uint32_t n_blocks, bool canon,
+                                                    uint32_t n_blocks,
                                                     const uint8_t *(&frac)[kChains],
                                                     const uint8_t *(&next_frac)[kChains], Sink &sink,
                                                     uint8_t *(&exp)[kChains], uint32_t ring) {
   constexpr uint32_t kFracStride = 32u * (S + 1);
   constexpr uint32_t kRingUnitBytes = ring_unit_bytes(S);
   constexpr uint32_t kRingSlotBytes = kChains * kRingUnitBytes;
-  // Blocks per trip of the unrolled loop.  Two: the code of a trip (about 4 KB a block) is
+  // Blocks per trip of the loop over the ring.  Two: the code of a trip (about 4 KB a block) is
   // fetched once per SM, which a call that decodes one group per warp pays for in full.
-  // Tables in the wide layout (unusual alphabets) take one block per trip.
-  constexpr int kTrip = ROW > 0 ? 2 : 1;
+  constexpr int kTrip = 2;
   if (!MERGE) {
 #pragma unroll 1
     for (uint32_t b = 0; b < n_blocks; ++b) {
@@ -456,7 +456,7 @@ __device__ __forceinline__ bool decode_blocks_multi(LaneState (&st)[kChains], co
 #pragma unroll
       for (int c = 0; c < C; ++c) {
         w[c][t] = merge_word<S, ROW>(e0[c], e1[c], bits[c], t);
-        if (ROW == 0 && canon) w[c][t] = canon_word(w[c][t]);
+        if (CANON) w[c][t] = canon_word(w[c][t]);
       }
     }
 #pragma unroll
@@ -474,42 +474,40 @@ __device__ __forceinline__ bool decode_blocks_multi(LaneState (&st)[kChains], co
     // (`fetch`: where that block's fractions are).  When the group fills the ring a whole
     // number of times, the copies go on after its last block with the first three of the next
     // group (next_frac, unless null), which finds them where ring_prologue would put them.
-    const bool carry = kTrip > 1 && n_blocks && n_blocks % kRingSlots == 0 && next_frac[0] != nullptr;
+    const bool carry = n_blocks && n_blocks % kRingSlots == 0 && next_frac[0] != nullptr;
     uint32_t b = 0;
     const uint8_t *fetch[kChains];
 #pragma unroll
     for (int c = 0; c < C; ++c) fetch[c] = frac[c] + 3 * kFracStride;
-    if (kTrip > 1) {
-      const uint32_t fetch_end = carry ? ~0u : n_blocks;
-      uint32_t half = 0;                       // byte offset of the trip's two ring slots
+    const uint32_t fetch_end = carry ? ~0u : n_blocks;
+    uint32_t half = 0;                       // byte offset of the trip's two ring slots
 #pragma unroll 1
-      for (; b + kTrip <= n_blocks; b += kTrip) {
-        uint64_t bits[kChains];
-        if (b + 3 < fetch_end) {
+    for (; b + kTrip <= n_blocks; b += kTrip) {
+      uint64_t bits[kChains];
+      if (b + 3 < fetch_end) {
 #pragma unroll
-          for (int c = 0; c < C; ++c)
-            frac_async<S>(ring + (half ^ (2 * kRingSlotBytes)) + kRingSlotBytes + c * kRingUnitBytes,
-                          fetch[c]);
-        }
-        ring_read(half, bits);
-        decode_block(bits, 0);
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-          fetch[c] += kFracStride;
-          if (carry && b + 4 == n_blocks) fetch[c] = next_frac[c];
-        }
-        if (b + 4 < fetch_end) {
-#pragma unroll
-          for (int c = 0; c < C; ++c)
-            frac_async<S>(ring + half + c * kRingUnitBytes, fetch[c]);
-        }
-        ring_read(half + kRingSlotBytes, bits);
-        decode_block(bits, 1);
-#pragma unroll
-        for (int c = 0; c < C; ++c) fetch[c] += kFracStride;
-        half ^= 2 * kRingSlotBytes;
-        sink.advance(kTrip);
+        for (int c = 0; c < C; ++c)
+          frac_async<S>(ring + (half ^ (2 * kRingSlotBytes)) + kRingSlotBytes + c * kRingUnitBytes,
+                        fetch[c]);
       }
+      ring_read(half, bits);
+      decode_block(bits, 0);
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        fetch[c] += kFracStride;
+        if (carry && b + 4 == n_blocks) fetch[c] = next_frac[c];
+      }
+      if (b + 4 < fetch_end) {
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+          frac_async<S>(ring + half + c * kRingUnitBytes, fetch[c]);
+      }
+      ring_read(half + kRingSlotBytes, bits);
+      decode_block(bits, 1);
+#pragma unroll
+      for (int c = 0; c < C; ++c) fetch[c] += kFracStride;
+      half ^= 2 * kRingSlotBytes;
+      sink.advance(kTrip);
     }
 #pragma unroll 1
     for (; b < n_blocks; ++b) {
@@ -529,52 +527,41 @@ __device__ __forceinline__ bool decode_blocks_multi(LaneState (&st)[kChains], co
     return carry;
   }
   // Narrow fractions: a double-buffered ring filled one group of four blocks ahead; lanes
-  // then read their own 1 or 2 bytes.
-  uint32_t b = 0;
-  if (ring_by_group(S, n_blocks)) {
-    const uint32_t lane_id = threadIdx.x & 31;
-    const uint32_t ring0 = ring - lane_id * 4;             // `ring` carries lane*4 for s<7
-    const uint32_t n_groups = n_blocks >> 2;
+  // then read their own 1 or 2 bytes.  Only the one to three blocks behind the last whole group
+  // (43 blocks a unit in matrices with 11008 columns) are loaded into registers: the chain's
+  // lookups wait for such loads.
+  const uint32_t lane_id = threadIdx.x & 31;
+  const uint32_t ring0 = ring - lane_id * 4;               // `ring` carries lane*4 for s<7
+  const uint32_t n_groups = n_blocks >> 2;
 #pragma unroll 1
-    for (uint32_t g = 0; g < n_groups; ++g) {
-      __syncwarp();                       // everyone is done with the buffer about to be refilled
-      if (g + 1 < n_groups) {
-        group_async<S, C>(ring, frac, g + 1);
-        frac_wait<1>();
-      } else {
-        frac_wait<0>();
-      }
-      __syncwarp();                       // all lanes' copies of group g have landed
-      const uint32_t src = ring0 + (g & 1) * kRingSlotBytes + lane_id * (S + 1);
-      auto group_block = [&](int at, int k) {
-        uint64_t bits[kChains];
-#pragma unroll
-        for (int c = 0; c < C; ++c)
-          bits[c] = (S == 1) ? lds_u16(src + c * kRingUnitBytes + at * 64)
-                             : lds_u8(src + c * kRingUnitBytes + at * 32);
-        decode_block(bits, k);
-      };
-#pragma unroll 1
-      for (int at = 0; at < 4; at += kTrip) {
-#pragma unroll
-        for (int k = 0; k < kTrip; ++k) group_block(at + k, k);
-        sink.advance(kTrip);
-      }
+  for (uint32_t g = 0; g < n_groups; ++g) {
+    __syncwarp();                         // everyone is done with the buffer about to be refilled
+    if (g + 1 < n_groups) {
+      group_async<S, C>(ring, frac, g + 1);
+      frac_wait<1>();
+    } else {
+      frac_wait<0>();
     }
-    return false;
-  }
-  uint64_t next[kChains];
-#pragma unroll
-  for (int c = 0; c < C; ++c) next[c] = load_frac<S>(frac[c]);
+    __syncwarp();                         // all lanes' copies of group g have landed
+    const uint32_t src = ring0 + (g & 1) * kRingSlotBytes + lane_id * (S + 1);
+    // one block per trip: with two, the lone warp's step takes 119 instead of 85 cycles at
+    // precision 0, and 115 instead of 87 at precision 1
 #pragma unroll 1
-  for (; b < n_blocks; ++b) {
+    for (int at = 0; at < 4; ++at) {
+      uint64_t bits[kChains];
+#pragma unroll
+      for (int c = 0; c < C; ++c)
+        bits[c] = (S == 1) ? lds_u16(src + c * kRingUnitBytes + at * 64)
+                           : lds_u8(src + c * kRingUnitBytes + at * 32);
+      decode_block(bits, 0);
+      sink.advance(1);
+    }
+  }
+#pragma unroll 1
+  for (uint32_t b = n_groups * 4; b < n_blocks; ++b) {
     uint64_t bits[kChains];
 #pragma unroll
-    for (int c = 0; c < C; ++c) {
-      bits[c] = next[c];
-      frac[c] += kFracStride;
-      if (b + 1 < n_blocks) next[c] = load_frac<S>(frac[c]);
-    }
+    for (int c = 0; c < C; ++c) bits[c] = load_frac<S>(frac[c] + b * kFracStride);
     decode_block(bits, 0);
     sink.advance(1);
   }
@@ -595,7 +582,10 @@ __device__ __forceinline__ void decode_rest(const DecodeArgs &a, LaneState &st, 
   uint16_t *out_lane = MERGE ? a.out_bf16 + ((int64_t)unit_out_index(a, u, lane) + delta) : nullptr;
   uint8_t *exp_lane = MERGE ? nullptr : a.out_exp + ((int64_t)e_lane + delta);
   const uint32_t adv = (MERGE && a.tile_cols) ? 64u : 256u;
-  decode_blocks<S, MERGE>(a, st, lv, b0, full_blocks, e_lane, out_lane, exp_lane, adv, canon);
+  if (lv.narrow)
+    decode_blocks<S, MERGE, kNarrowRow>(a, st, lv, b0, full_blocks, e_lane, out_lane, exp_lane, adv, canon);
+  else
+    decode_blocks<S, MERGE, 0>(a, st, lv, b0, full_blocks, e_lane, out_lane, exp_lane, adv, canon);
   if (count == U) {
     if (__any_sync(0xFFFFFFFFu, st.x != kStateLow) && lane == 0)
       raise(a.status, NZ_STATUS_BAD_STATE);
@@ -603,7 +593,7 @@ __device__ __forceinline__ void decode_rest(const DecodeArgs &a, LaneState &st, 
     const uint64_t e0 = e_lane + (uint64_t)full_blocks * 256;
 #pragma unroll 1
     for (int t = 0; t < 8; ++t) {
-      const uint32_t ent = decode_step<kAnyRow>(st, lv);
+      const uint32_t ent = decode_step_any(st, lv);
       emit_guarded<S, MERGE>(entry_symbol(ent), e0 + t, delta, a);
     }
   }
@@ -792,19 +782,26 @@ __device__ __forceinline__ void dot_single(const DecodeArgs &a, const UnitPlan &
       const uint8_t *frac_lane = a.frac + (first + lane * 8) * (S + 1) / 8;
       DotLane d;
       d.start(a.gx, a.in, first, part, lane);
-      for (uint32_t b = 0; b < n_blocks; ++b) {
-        const uint64_t fbits = load_frac<S>(frac_lane + (uint64_t)b * 32u * (S + 1));
-        uint32_t ent[8], w[4];
-        d.begin();
+      auto blocks = [&](auto row) {
+        uint64_t next = load_frac<S>(frac_lane);
+#pragma unroll 1
+        for (uint32_t b = 0; b < n_blocks; ++b) {
+          const uint64_t fbits = next;
+          if (b + 1 < n_blocks) next = load_frac<S>(frac_lane += 32u * (S + 1));
+          uint32_t ent[8], w[4];
+          d.begin();
 #pragma unroll
-        for (int t = 0; t < 8; ++t) ent[t] = decode_step<kAnyRow>(st, lv);
+          for (int t = 0; t < 8; ++t) ent[t] = decode_step<decltype(row)::value>(st, lv);
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          w[t] = merge_word<S>(ent[2 * t], ent[2 * t + 1], fbits, t);
-          if (canon) w[t] = canon_word(w[t]);
+          for (int t = 0; t < 4; ++t) {
+            w[t] = merge_word<S>(ent[2 * t], ent[2 * t + 1], fbits, t);
+            if (canon) w[t] = canon_word(w[t]);
+          }
+          d.put(w);
         }
-        d.put(w);
-      }
+      };
+      if (lv.narrow) blocks(std::integral_constant<int, kNarrowRow>());
+      else blocks(std::integral_constant<int, 0>());
       d.finish();
       if (count == U && __any_sync(0xFFFFFFFFu, st.x != kStateLow) && lane == 0)
         raise(a.status, NZ_STATUS_BAD_STATE);
@@ -1093,21 +1090,17 @@ decode_kernel(const BatchArgs batch) {
           xb[c] = MERGE ? nullptr : a.out_exp + o;
           init_sink(sink, c, a, real[c], o, lane);
         }
-        if (DOT || UPDATE || chains == kChains) {
-          if (lv.narrow && row_shift == kFastRow)
-            primed = decode_blocks_multi<S, MERGE, kFastRow, kChains>(st, lv, common, false, fr, nfr, sink, xb, ring);
-          else if (S != 7 && lv.narrow)            // kFastRow - 1, see narrow_rows
-            primed = decode_blocks_multi<S, MERGE, kFastRow - 1, kChains>(st, lv, common, false, fr, nfr, sink, xb, ring);
-          else
-            primed = decode_blocks_multi<S, MERGE, 0, kChains>(st, lv, common, canon, fr, nfr, sink, xb, ring);
-        } else {
-          if (lv.narrow && row_shift == kFastRow)
-            primed = decode_blocks_multi<S, MERGE, kFastRow, 1>(st, lv, common, false, fr, nfr, sink, xb, ring);
-          else if (S != 7 && lv.narrow)
-            primed = decode_blocks_multi<S, MERGE, kFastRow - 1, 1>(st, lv, common, false, fr, nfr, sink, xb, ring);
-          else
-            primed = decode_blocks_multi<S, MERGE, 0, 1>(st, lv, common, canon, fr, nfr, sink, xb, ring);
-        }
+        auto with = [&](auto cc) {
+          constexpr int C = decltype(cc)::value;
+#define NZ_LOOP(ROW, CANON) decode_blocks_multi<S, MERGE, ROW, CANON, C>(st, lv, common, fr, nfr, sink, xb, ring)
+          if (lv.narrow && row_shift == kFastRow) primed = NZ_LOOP(kFastRow, false);
+          else if (S != 7 && lv.narrow) primed = NZ_LOOP(kFastRow - 1, false);     // see narrow_rows
+          else if (MERGE && canon) primed = NZ_LOOP(0, true);
+          else primed = NZ_LOOP(0, false);
+#undef NZ_LOOP
+        };
+        if (DOT || UPDATE || chains == kChains) with(std::integral_constant<int, kChains>());
+        else with(std::integral_constant<int, 1>());
         finish_sink(sink);
       };
       if (DOT) {

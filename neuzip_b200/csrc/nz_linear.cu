@@ -185,7 +185,7 @@ struct LinChain {
 __device__ __forceinline__ void chain_symbols(LinChain &ch, const LutView &lv, uint32_t (&ent)[8]) {
   if (ch.kind == kUnitCoded) {
 #pragma unroll
-    for (int t = 0; t < 8; ++t) ent[t] = decode_step<kAnyRow>(ch.st, lv);
+    for (int t = 0; t < 8; ++t) ent[t] = decode_step_any(ch.st, lv);
   } else {
     // units start on any 16-bit word of the payload
     const uint16_t *src = reinterpret_cast<const uint16_t *>(ch.raw);
