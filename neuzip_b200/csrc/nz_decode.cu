@@ -55,32 +55,37 @@ static inline uint64_t work_units(const HostItem &it) {
   return it.unit_list ? it.n_list : unit_count(it.n, it.S);
 }
 
-// Cycles per symbol step of a CTA whose `w` warps decode two chains each, with `copies`
-// copies of the table: the latency of the dependent chain, or what its four schedulers
-// (17 cycles per warp-symbol) or its shared-memory pipe (2.7 wavefronts and one table
-// lookup, in which 32 / copies lanes share a bank) need.  Without a loop for narrow rows
-// (`narrow` false) the chains of a warp hardly overlap.
-//
-// A tensor with so few units that every one can have a warp of its own (20 per SM) is decoded
-// with one chain per warp instead of two: a step then takes the latency of one chain (73
-// cycles on a B200, 107 with two chains in a lone warp), on twice as many warps.
-static uint32_t step_cycles(uint32_t w, uint32_t copies, bool narrow) {
-  const uint32_t issue = (narrow ? 34 : 40) * ((w + 3) / 4);
-  const uint32_t wavefronts10 = 27 + (copies >= 32 ? 10 : copies >= 16 ? 20 : copies >= 8 ? 35 : 50);
-  const uint32_t lsu = 2 * w * wavefronts10 / 10;
-  const uint32_t latency = narrow ? 84 : 150;
-  uint32_t t = issue > lsu ? issue : lsu;
-  return t > latency ? t : latency;
+// Cycles per symbol step of a CTA with `w` warps of `chains` units each, as measured on a B200
+// (units of 256 to 512 symbols, one warp to twenty): the latency of the dependent chains while
+// a scheduler has one warp or two, then what the schedulers' integer pipes need.  Without a
+// loop for narrow rows (`narrow` false) a step has one instruction more and a longer chain, and
+// beside the smallest table (`smallest`) more of its lookups meet in a bank.  The merge of
+// precisions 0 and 1 is the cheapest.
+static uint32_t step_cycles(uint32_t w, uint32_t chains, bool narrow, bool smallest, int precision) {
+  uint32_t t;
+  if (chains == 1) {
+    t = (narrow ? 65 : 75) + (w > 8 ? 5 * (w - 8) : 0);
+  } else if (w <= 4) {
+    t = narrow ? 90 : 98;
+  } else {
+    const uint32_t slope10 = precision < 3 ? 84 : narrow ? 95 : 104;
+    t = (narrow || precision < 3 ? 111 : 119) + (w > 8 ? slope10 * (w - 8) / 10 : 0);
+  }
+  return smallest ? t + t / 20 : t;
 }
 
 // Grid geometry of one launch over `count` tensors.  One CTA per SM.  Every
-// warp decodes whole units, kChains at a time, so a tensor is only as fast as its
-// busiest CTA, and a CTA whose groups of units are not a multiple of its warps ends on a
-// round that few warps share.  Tensors of one launch differ in size and in unit length: each
-// gets its own number of warps (as many as its units leave room for) and of CTAs -- in
-// proportion to the symbols first, then moved one at a time from the tensor that finishes
-// first to the one that finishes last, by the estimate of step_cycles.  The number of table
-// copies is the one with the lowest estimate for the busiest CTA.
+// warp decodes whole units, so a tensor is only as fast as its busiest CTA.  A tensor with so
+// few units that every one can have a warp of its own is decoded with one chain per warp: a
+// step then takes the latency of one chain (65 cycles instead of 90 in a lone warp).  Others are
+// decoded kChains units at a time, by no more warps than make the rounds even (14 groups and 13
+// warps: two rounds of 7).  Tensors of one launch differ in size and in unit length: each gets its
+// own number of warps and of CTAs -- in proportion to the symbols first, then moved one at a time
+// from the tensor that finishes first to the one that finishes last, by the estimate of
+// step_cycles.  The number of table copies is the one with the lowest estimate for the busiest
+// CTA: more copies than one per two banks do not speed a step up, but they take the place of
+// warps, and with fewer there is no loop for narrow rows (8192 x 8192 elements at precision 0: 14
+// warps beside 8 copies 48 us, 7 warps twice beside 16 copies 58).
 static int decode_geometry(const HostItem *items, uint32_t count, int precision, uint32_t ring_bytes,
                            BatchArgs &b, uint32_t &warps, uint32_t &smem_bytes) {
   const uint32_t sm_smem = 227u * 1024u;
@@ -117,6 +122,14 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
     share[t] = (uint32_t)c;
     used += share[t];
   }
+  // units of a CTA, and whether each of them gets a warp beside a table of 4096 << sh bytes
+  // (matrix-vector and update launches always decode two units per warp)
+  const bool pairs_only = items[0].gx || items[0].grad;
+  auto own = [&](uint32_t t, uint32_t c) { return (uint32_t)((work_units(items[t]) + c - 1) / c); };
+  auto alone = [&](uint32_t t, uint32_t units, uint32_t sh) {
+    return !pairs_only && units <= max_warps &&
+           (4096u << sh) + guard[t] + units * (b.item[t].slot_bytes + ring_bytes) <= sm_smem;
+  };
   const uint32_t pb = usual_prob_bits(precision);
   uint64_t best = ~0ull;
   uint32_t ctas[kMaxBatch] = {};
@@ -135,11 +148,13 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
     }
     if (!fits) continue;
     auto cost = [&](uint32_t t, uint32_t c) -> uint64_t {
-      const uint32_t g = (groups[t] + c - 1) / c;
-      const uint32_t full = g / cap[t], rest = g - full * cap[t];
-      return (uint64_t)items[t].S *
-             ((uint64_t)full * step_cycles(cap[t], copies, narrow) +
-              (rest ? step_cycles(rest, copies, narrow) : 0));
+      const uint32_t units = own(t, c);
+      if (alone(t, units, sh)) return (uint64_t)items[t].S * step_cycles(units, 1, narrow, sh == 2, precision);
+      const uint32_t g = (groups[t] + c - 1) / c, rounds = (g + cap[t] - 1) / cap[t];
+      // between two rounds a warp opens its next units
+      constexpr uint32_t kRoundCycles = 1500;
+      const uint32_t step = step_cycles((g + rounds - 1) / rounds, kChains, narrow, sh == 2, precision);
+      return (uint64_t)rounds * (items[t].S * step + kRoundCycles);
     };
     uint32_t now[kMaxBatch], sum = used;
     for (uint32_t t = 0; t < count; ++t) now[t] = share[t];
@@ -175,8 +190,7 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
     // small launch has
     uint64_t worst = 0;
     for (uint32_t t = 0; t < count; ++t) {
-      const uint64_t own = (work_units(items[t]) + now[t] - 1) / now[t];
-      const uint32_t writers = own < 4 && own < cap[t] ? (uint32_t)own : 4;
+      const uint32_t units = own(t, now[t]), writers = units < 4 ? units : 4;
       const uint64_t c = cost(t, now[t]) + (4096u << sh) / (16 * writers);
       if (c > worst) worst = c;
     }
@@ -198,12 +212,10 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
     // no more warps than make the rounds even, and a second staging buffer per warp where
     // there is more than one round and room for it
     const uint64_t units = work_units(items[t]);
-    const uint32_t own = (uint32_t)((units + ctas[t] - 1) / ctas[t]);     // units per CTA
     const uint32_t fixed0 = b.lut_bytes + guard[t];
-    if (!items[0].gx && !items[0].grad && own <= max_warps &&
-        fixed0 + own * (it.slot_bytes + ring_bytes) <= sm_smem) {
+    if (alone(t, own(t, ctas[t]), b.lut_shift)) {
       it.chains = 1;
-      it.warps = own;
+      it.warps = own(t, ctas[t]);
       it.bufs = 1;
       it.groups_each = (uint32_t)units / (ctas[t] * it.warps);
       it.groups_more = (uint32_t)units % (ctas[t] * it.warps);
