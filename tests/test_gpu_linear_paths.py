@@ -53,20 +53,25 @@ def test_raw_units_between_coded_ones(s):
 
 @pytest.mark.parametrize("m", (1, 17, 256))
 @pytest.mark.parametrize("cols,S", ((2048, 128), (11008, 344), (4096, 256)))
-def test_with_and_without_room_for_the_rings(cols, S, m):
+@pytest.mark.parametrize("nan", (False, True))
+def test_with_and_without_room_for_the_rings(cols, S, m, nan):
     rows = 260
     g = torch.Generator().manual_seed(cols + m)
     w = (torch.randn(rows, cols, generator=g) * 0.02).to(torch.bfloat16).cuda()
+    if nan:
+        w[7, 5] = float("nan")           # its row is NaN, the others take the loop that looks for it
     x = torch.randn(m, cols, generator=g).to(torch.bfloat16).cuda()
-    for s in (7, 3):
+    for s in (7, 3, 1, 0):
         cont, frac, mw = A.compress_operand(w, rows, cols, s, S)
         stored = A.decompress_operand(cont, frac, rows, cols, s, S)[0].view(rows, cols)
         if S == 344 and m == 256:
             continue                              # units too long beside this many input rows
         ys = []
         for _ in range(3):
-            y, status = A.linear(cont, frac, rows, cols, s, S, x, max_words=mw)
+            y, status = A.linear(cont, frac, rows, cols, s, S, x, max_words=mw, canon=nan)
             assert status == 0
             ys.append(y)
-        check(ys[0].cpu(), reference(stored.cpu(), x.cpu()))
-        assert all(torch.equal(ys[0], y) for y in ys)
+        lost = stored.isnan().any(1).cpu()            # (precision 0 rounds the NaN away)
+        check(ys[0].cpu()[:, ~lost], reference(stored.cpu(), x.cpu())[:, ~lost])
+        assert bool(ys[0].cpu()[:, lost].isnan().all()) and bool(lost.any()) == (nan and s > 0)
+        assert all(torch.equal(ys[0].view(torch.int16), y.view(torch.int16)) for y in ys)
