@@ -22,33 +22,27 @@ def check(y, ref):
     assert bool((err <= 2.0 ** -8 * ref.abs() + 2.0 ** -14 * ref.abs().max()).all())
 
 
-@pytest.mark.parametrize("s", (7, 3, 0))
+@pytest.mark.parametrize("s", (7, 3, 1, 0))
 def test_raw_units_between_coded_ones(s):
-    rows, cols, S = 132, 2048, 128
+    # the identity as input: every weight reaches one result, alone, so each has to be exact
+    rows, cols, S = 132, 1024, 64
     g = torch.Generator().manual_seed(s)
     w = (torch.randn(rows, cols, generator=g) * 0.02).to(torch.bfloat16)
     bits = A.to_bits(w).reshape(rows, cols).copy()
     rng = np.random.default_rng(3)
-    for row in (0, 20, 64, 100):                     # row groups whose exponents do not compress
-        bits[row:row + 4, :1024] = ((rng.integers(1, 250, (4, 1024)) << 7) | (bits[row:row + 4, :1024] & 0x807F))
-    bits[np.isin(bits >> 7 & 0xFF, (255,))] = 0
-    # keep the products finite: large exponents only against zero inputs
-    x = torch.randn(16, cols, generator=g).to(torch.bfloat16)
-    x[:, :1024] = 0
-    x[:, 7] = 2.0 ** -100
-    wt = A.from_bits(bits.reshape(-1))
-    cont, frac, mw = A.compress_operand(wt, rows, cols, s, S)
+    for row in range(0, rows, 12):                   # row groups whose exponents do not compress
+        bits[row:row + 4, :512] = ((rng.integers(1, 250, (4, 512)) << 7) | (bits[row:row + 4, :512] & 0x807F))
+    cont, frac, mw = A.compress_operand(A.from_bits(bits.reshape(-1)), rows, cols, s, S)
     offs = np.frombuffer(cont.cpu().numpy().tobytes(), dtype=np.uint32, count=rows // 4 * 2 + 1, offset=576)
     raw = offs[:-1] >> 31 == 1
-    assert raw.any() and not raw.all() and (offs[:-1][raw] & 1).any()     # some at odd words
-    stored = A.decompress_operand(cont, frac, rows, cols, s, S)[0].view(rows, cols)
-    y, status = A.linear(cont, frac, rows, cols, s, S, x.cuda(), max_words=mw)
+    assert list(np.flatnonzero(raw)) == list(range(0, rows // 2, 6))
+    assert (offs[:-1][raw] & 1).any() and not (offs[:-1][raw] & 1).all()      # at odd and even words
+    c_ref, f_ref = O.compress_bf16(O.to_operand_order(bits.reshape(-1), rows, cols), s, S)
+    stored = O.from_operand_order(O.decompress_bf16(c_ref, f_ref, bits.size, s), rows, cols)
+    y, status = A.linear(cont, frac, rows, cols, s, S, torch.eye(cols, dtype=torch.bfloat16, device="cuda"),
+                         max_words=mw)
     assert status == 0
-    keep = torch.ones(rows, dtype=torch.bool)
-    for row in (0, 20, 64, 100):
-        keep[row:row + 4] = False
-    check(y.cpu()[:, keep], reference(stored.cpu(), x)[:, keep])
-    check(y.cpu()[:, ~keep].clamp(-1e30, 1e30), reference(stored.cpu(), x)[:, ~keep].clamp(-1e30, 1e30))
+    assert torch.equal(y.cpu().t(), A.from_bits(stored, "cpu").view(rows, cols))
 
 
 @pytest.mark.parametrize("m", (1, 17, 256))
