@@ -96,11 +96,15 @@ def test_long_units_beyond_one_wave(S):
     check(bits_of("uniform10", 32 * S * (148 * 8 + 3) - 77, 12), 1, S)
 
 
-@pytest.mark.parametrize("units", (255, 256, 257, 148 * 48 * 3 + 4, 255 * 512 + 1))
+@pytest.mark.parametrize("units", (255, 256, 257, 148 * 48 * 3 + 4, 131071, 131072, 131072 + 300))
 def test_many_units(units):
-    # chunks of one and more units, several units per warp, and offsets from the scan kernel
+    # chunks of one and more units, several units per warp; from 131072 units on the offsets, the
+    # raw count and the largest unit come from the scan kernel
     n = 256 * units - 23
     bits = bits_of("peaked", n, 3)
-    cont, frac, _ = A.compress(A.from_bits(bits), 7, 8)
-    c_ref, f_ref = O.compress_bf16(bits, 7, 8)
-    assert np.array_equal(cont.cpu().numpy(), c_ref) and np.array_equal(frac.cpu().numpy(), f_ref)
+    raw = np.random.default_rng(4).integers(0, 256, 256 * 70).astype(np.uint16)
+    for first in (0, 100, units // 2, units - 80):          # some units that do not compress
+        bits[256 * first:256 * (first + 70)] = (raw << 7)[:max(0, n - 256 * first)]
+    cont = check(bits, 7, 8)
+    offs = np.frombuffer(cont.tobytes(), dtype=np.uint32, count=units, offset=576)
+    assert (offs >> 31).any() and not (offs >> 31).all()
