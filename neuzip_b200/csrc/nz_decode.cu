@@ -50,9 +50,9 @@ struct HostItem {
   uint32_t norm_lg;
 };
 
-// Units a launch decodes for an item.
-static inline uint64_t work_units(const HostItem &it) {
-  return it.unit_list ? it.n_list : unit_count(it.n, it.S);
+// Units a launch decodes for an item (a tensor has fewer than 2^24).
+static inline uint32_t work_units(const HostItem &it) {
+  return it.unit_list ? it.n_list : (uint32_t)unit_count(it.n, it.S);
 }
 
 // Cycles per symbol step of a CTA with `w` warps of `chains` units each, as measured on a B200
@@ -92,7 +92,7 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
   const uint32_t max_warps = items[0].gx ? (uint32_t)kDotMaxWarps
                              : items[0].grad ? (uint32_t)kUpdateMaxWarps : (uint32_t)NZ_DECODE_MAX_WARPS;
   uint64_t total_work = 0, total_units = 0;
-  uint32_t groups[kMaxBatch], guard[kMaxBatch], per_warp[kMaxBatch];
+  uint32_t units[kMaxBatch], groups[kMaxBatch], guard[kMaxBatch], per_warp[kMaxBatch];
   for (uint32_t t = 0; t < count; ++t) {
     const uint64_t U = 32ull * items[t].S;
     uint64_t ub = items[t].max_unit_words ? (uint64_t)items[t].max_unit_words * 2 : U;
@@ -105,8 +105,9 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
       set_error("decode: a warp's units of %u symbols do not fit in shared memory", (unsigned)U);
       return NZ_E_ARG;
     }
-    groups[t] = (uint32_t)((work_units(items[t]) + kChains - 1) / kChains);
-    total_units += work_units(items[t]);
+    units[t] = work_units(items[t]);         // at least one
+    groups[t] = (units[t] - 1) / kChains + 1;
+    total_units += units[t];
     total_work += (uint64_t)groups[t] * items[t].S;
   }
   // CTAs per tensor: one per SM (fewer when there is not enough work to give every SM a
@@ -117,7 +118,7 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
   uint32_t share[kMaxBatch], used = 0;
   for (uint32_t t = 0; t < count; ++t) {
     uint64_t c = total_work ? (uint64_t)groups[t] * items[t].S * n_ctas / total_work : 1;
-    if (c > work_units(items[t])) c = work_units(items[t]);
+    if (c > units[t]) c = units[t];
     if (c < 1) c = 1;
     share[t] = (uint32_t)c;
     used += share[t];
@@ -125,10 +126,10 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
   // units of a CTA, and whether each of them gets a warp beside a table of 4096 << sh bytes
   // (matrix-vector and update launches always decode two units per warp)
   const bool pairs_only = items[0].gx || items[0].grad;
-  auto own = [&](uint32_t t, uint32_t c) { return (uint32_t)((work_units(items[t]) + c - 1) / c); };
-  auto alone = [&](uint32_t t, uint32_t units, uint32_t sh) {
-    return !pairs_only && units <= max_warps &&
-           (4096u << sh) + guard[t] + units * (b.item[t].slot_bytes + ring_bytes) <= sm_smem;
+  auto own = [&](uint32_t t, uint32_t c) { return (units[t] - 1) / c + 1; };
+  auto alone = [&](uint32_t t, uint32_t each, uint32_t sh) {
+    return !pairs_only && each <= max_warps &&
+           (4096u << sh) + guard[t] + each * (b.item[t].slot_bytes + ring_bytes) <= sm_smem;
   };
   const uint32_t pb = usual_prob_bits(precision);
   uint64_t best = ~0ull;
@@ -148,8 +149,8 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
     }
     if (!fits) continue;
     auto cost = [&](uint32_t t, uint32_t c) -> uint64_t {
-      const uint32_t units = own(t, c);
-      if (alone(t, units, sh)) return (uint64_t)items[t].S * step_cycles(units, 1, narrow, sh == 2, precision);
+      const uint32_t each = own(t, c);
+      if (alone(t, each, sh)) return (uint64_t)items[t].S * step_cycles(each, 1, narrow, sh == 2, precision);
       const uint32_t g = (groups[t] + c - 1) / c, rounds = (g + cap[t] - 1) / cap[t];
       // between two rounds a warp opens its next units
       constexpr uint32_t kRoundCycles = 1500;
@@ -166,7 +167,7 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
         for (uint32_t t = 1; t < count; ++t)
           if (cost(t, now[t]) > cost(hi, now[hi])) hi = t;
         if (sum < n_ctas) {
-          if (now[hi] >= work_units(items[hi])) break;
+          if (now[hi] >= units[hi]) break;
           ++now[hi];
           ++sum;
           continue;
@@ -181,7 +182,7 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
           --sum;
           continue;
         }
-        if (now[hi] >= work_units(items[hi]) || cost(lo, now[lo] - 1) >= cost(hi, now[hi])) break;
+        if (now[hi] >= units[hi] || cost(lo, now[lo] - 1) >= cost(hi, now[hi])) break;
         --now[lo];
         ++now[hi];
       }
@@ -190,7 +191,7 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
     // small launch has
     uint64_t worst = 0;
     for (uint32_t t = 0; t < count; ++t) {
-      const uint32_t units = own(t, now[t]), writers = units < 4 ? units : 4;
+      const uint32_t each = own(t, now[t]), writers = each < 4 ? each : 4;
       const uint64_t c = cost(t, now[t]) + (4096u << sh) / (16 * writers);
       if (c > worst) worst = c;
     }
@@ -211,14 +212,13 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
     BatchItem &it = b.item[t];
     // no more warps than make the rounds even, and a second staging buffer per warp where
     // there is more than one round and room for it
-    const uint64_t units = work_units(items[t]);
-    const uint32_t fixed0 = b.lut_bytes + guard[t];
-    if (alone(t, own(t, ctas[t]), b.lut_shift)) {
+    const uint32_t fixed0 = b.lut_bytes + guard[t], each = own(t, ctas[t]);
+    if (alone(t, each, b.lut_shift)) {
       it.chains = 1;
-      it.warps = own(t, ctas[t]);
+      it.warps = each;
       it.bufs = 1;
-      it.groups_each = (uint32_t)units / (ctas[t] * it.warps);
-      it.groups_more = (uint32_t)units % (ctas[t] * it.warps);
+      it.groups_each = units[t] / (ctas[t] * it.warps);
+      it.groups_more = units[t] % (ctas[t] * it.warps);
     } else {
       const uint32_t g = (groups[t] + ctas[t] - 1) / ctas[t];
       const uint32_t rounds = (g + it.warps - 1) / it.warps;
