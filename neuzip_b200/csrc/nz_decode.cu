@@ -90,7 +90,7 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
                            BatchArgs &b, uint32_t &warps, uint32_t &smem_bytes) {
   const uint32_t sm_smem = 227u * 1024u;
   const uint32_t max_warps = items[0].gx ? (uint32_t)kDotMaxWarps
-                             : items[0].grad ? (uint32_t)kUpdateMaxWarps : (uint32_t)NZ_DECODE_MAX_WARPS;
+                             : items[0].grad ? (uint32_t)kUpdateMaxWarps : (uint32_t)kDecodeMaxWarps;
   uint64_t total_work = 0, total_units = 0;
   uint32_t units[kMaxBatch], groups[kMaxBatch], guard[kMaxBatch], per_warp[kMaxBatch];
   for (uint32_t t = 0; t < count; ++t) {
@@ -259,7 +259,6 @@ int decode_many(const HostItem *items, uint32_t count, int precision, uint32_t S
     b.status = (uint32_t *)status;
     for (uint32_t t = 0; t < n_live; ++t) {
       b.item[t].container = (const uint8_t *)live[t].container;
-      b.item[t].container_bytes = live[t].container_bytes;
       b.item[t].frac = (const uint8_t *)live[t].frac;
       b.item[t].n = live[t].n;
       b.item[t].out_bf16 = (uint16_t *)live[t].out_bf16;

@@ -6,10 +6,6 @@
 
 #include "nz_common.cuh"
 
-#ifndef NZ_DECODE_CHAINS
-#define NZ_DECODE_CHAINS 2
-#endif
-
 namespace nz {
 
 // A wait is a bounded number of tries; each may suspend the thread for up to kWaitHintNs, so
@@ -95,15 +91,14 @@ struct LutView {
 //           9-bit table always has and weights at any resolution do too.
 // Either way one byte permutation puts the symbols of two entries where the exponents of
 // an output word's two bf16 go.  With the narrow layout frequency and offset are one
-// operation each and the state update needs no correction term: 12 instead of 13
-// instructions per symbol.  The loop is bound by the integer (ALU) pipe, which takes an
-// instruction every other cycle, next to instruction issue; on a B200 with 20 warps of two
-// chains a warp-symbol costs 16.4 cycles of a scheduler (17.2 with the wide layout).
+// operation each and the state update needs no correction term: 11 instead of 12
+// instructions per symbol.  Measured on a B200 with units of 256 symbols, two chains a warp:
+// 86 instead of 98 cycles a step in a lone warp, 226 instead of 242 with 20 warps (there the
+// integer pipe and the memory are both nearly full).
 constexpr uint32_t kEntSymShift = 23;
 constexpr uint32_t kEntFreqShift = 12;
 constexpr uint32_t kNarrowOffShift = 23;
 constexpr uint32_t kNarrowSymShift = 15;
-constexpr uint32_t kNarrowFreqMask = (1u << kNarrowSymShift) - 1u;
 constexpr uint32_t kNarrowMaxFreq = 512;
 // Resolution of the usual tables of a precision (up to 32 distinct exponents), the only one
 // with a loop for narrow entries.
@@ -217,17 +212,6 @@ __device__ __forceinline__ uint32_t merge_pair_generic(uint32_t ea, uint32_t eb,
   return out[0] | (out[1] << 16);
 }
 
-// Field of element j (0..7) of a lane's block; `bits` holds the lane's
-// (s+1) bytes of packed fractions, first byte in the low bits.
-template <int S>
-__device__ __forceinline__ uint32_t field_of(uint64_t bits, int j) {
-  constexpr int FB = S + 1;
-  const int bit = j * FB;                 // MSB-first position inside the byte string
-  const int byte = bit >> 3;
-  const int shift = 7 - S - (bit & 7);
-  return (uint32_t)(bits >> (8 * byte + shift)) & ((1u << FB) - 1u);
-}
-
 // Lossless fast path: two entries + two fraction bytes -> one 32-bit word.
 //   sel picks the two fraction bytes (a in both low bytes, b in both high).
 // Two bytes of each entry hold its exponent in place.
@@ -307,7 +291,6 @@ __device__ __forceinline__ uint32_t canon_word(uint32_t w) {
 
 struct DecodeArgs {
   const uint8_t *container;
-  uint64_t container_bytes;
   const uint8_t *frac;
   uint64_t n;
   uint32_t S;
@@ -318,7 +301,6 @@ struct DecodeArgs {
   uint32_t slot_bytes;
   uint32_t lut_shift;   // log2 of the bytes per slot row for a 2^12-slot table (2..5)
   uint32_t lut_bytes;   // 4096 << lut_shift
-  uint32_t ring_offset; // byte offset of the fraction rings in shared memory
   int canon;
   uint16_t *out_bf16;
   uint8_t *out_exp;
@@ -419,7 +401,7 @@ __device__ __forceinline__ uint64_t frac_from_ring(uint32_t addr) {
   return lds_u32(addr);
 }
 
-constexpr int kChains = NZ_DECODE_CHAINS;        // units a warp decodes side by side
+constexpr int kChains = 2;                       // units a warp decodes side by side
 
 constexpr uint32_t kRingSlots = 4;               // blocks of fractions in flight per unit + 1
 // Shared-memory ring of a warp for the packed fractions, by precision.  One unit's

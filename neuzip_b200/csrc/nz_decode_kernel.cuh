@@ -8,21 +8,21 @@
 // fractions straight into the bf16 output, so the exponent stream never makes
 // the round trip through HBM.
 //
-// Work decomposition.  One CTA per SM; a warp decodes kChains units side by
-// side (32 lane streams of S symbols each: the independent rANS chains hide one
-// another's latency).  The units' coded bytes are staged into the warp's
-// shared-memory slots with bulk asynchronous copies (cp.async.bulk + mbarrier,
+// Work decomposition.  One CTA per SM; a warp decodes a run of units, two side by side (32
+// lane streams of S symbols each: independent rANS chains hide one another's latency), or one
+// where every unit of the CTA can have a warp of its own.  The units' coded bytes are staged
+// into the warp's shared-memory slots with bulk asynchronous copies (cp.async.bulk + mbarrier,
 // no multicast); each lane then walks its own stream with a private read
 // pointer, so a renormalisation costs one predicated 16-bit shared load and no
 // warp-wide vote.  A lane produces 8 consecutive tensor elements per block and
 // writes them with one 128-bit store; the warp's stores are 512 contiguous
 // bytes.  The same kernel, instantiated differently, decodes a list of units
-// (gather) or feeds the decoded words to a dot product instead of a store.
+// (gather), feeds the decoded words to a dot product or applies an optimiser step to them.
 //
-// Decode table.  One 32-bit entry per slot (symbol << 23 | freq << 12 | offset
-// inside the symbol's slot range), built once per CTA from the container's
-// frequency table.  Random table lookups by 32 lanes would collide in the 32
-// shared-memory banks (3.5 wavefronts per lookup on average, which made the
+// Decode table.  One 32-bit entry per slot, built once per CTA from the container's
+// frequency table, in one of two layouts (see decode_step): narrow entries where the
+// frequencies allow it, wide ones otherwise.  Random table lookups by 32 lanes would collide
+// in the 32 shared-memory banks (3.5 wavefronts per lookup on average, which made the
 // shared-memory pipe the limiter), so the table is replicated across banks as
 // far as the shared memory left by the slots allows (64 KB for lossless
 // tensors: 32 copies of a 2^9-slot table, one per bank; 16 of a 2^10-slot one).
@@ -37,16 +37,11 @@
 
 #include <cuda_bf16.h>
 #include <string.h>
+
 #include <mutex>
 #include <type_traits>
 
 #include "nz_decode_core.cuh"
-
-// Tuning constants (measured on B200, lossless 7B-shape blocks): two units per warp
-// and 20 warps per CTA beat three units with 14-16 warps by 3 %.
-#ifndef NZ_DECODE_MAX_WARPS
-#define NZ_DECODE_MAX_WARPS (NZ_DECODE_CHAINS == 2 ? 20 : 16)
-#endif
 
 namespace nz {
 
@@ -54,9 +49,9 @@ namespace nz {
 // CTAs (one CTA per SM), sized in proportion to its unit count, so a small
 // tensor does not leave most of the machine idle.
 constexpr uint32_t kMaxBatch = 8;
+constexpr int kDecodeMaxWarps = 20;                  // 96 registers a thread: more of them would spill
 struct BatchItem {
   const uint8_t *container;
-  uint64_t container_bytes;
   const uint8_t *frac;
   uint64_t n;
   uint16_t *out_bf16;
@@ -820,9 +815,9 @@ __device__ __forceinline__ void dot_single(const DecodeArgs &a, const UnitPlan &
 // elements are multiplied with the input vector as they are decoded.
 constexpr int kModeTensor = 0, kModeList = 1, kModeDot = 2, kModeUpdate = 3;
 constexpr int kUpdateMaxWarps = 16;                 // the update's operands want registers
-constexpr int kDotMaxWarps = NZ_DECODE_MAX_WARPS;   // 16 warps and 128 registers measured slower
+constexpr int kDotMaxWarps = kDecodeMaxWarps;   // 16 warps and 128 registers measured slower
 template <int S, bool MERGE, int MODE>
-__global__ void __launch_bounds__((MODE == kModeDot ? kDotMaxWarps : MODE == kModeUpdate ? kUpdateMaxWarps : NZ_DECODE_MAX_WARPS) * 32, 1)
+__global__ void __launch_bounds__((MODE == kModeDot ? kDotMaxWarps : MODE == kModeUpdate ? kUpdateMaxWarps : kDecodeMaxWarps) * 32, 1)
 decode_kernel(const BatchArgs batch) {
   constexpr bool LIST = MODE == kModeList;
   constexpr bool DOT = MODE == kModeDot;
@@ -838,7 +833,6 @@ decode_kernel(const BatchArgs batch) {
   const uint32_t cta_rank = blockIdx.x - cta_first, cta_count = cta_end - cta_first;
   DecodeArgs a;
   a.container = batch.item[ti].container;
-  a.container_bytes = batch.item[ti].container_bytes;
   a.frac = batch.item[ti].frac;
   a.n = batch.item[ti].n;
   a.S = batch.item[ti].S;
@@ -849,7 +843,6 @@ decode_kernel(const BatchArgs batch) {
   a.slot_bytes = batch.item[ti].slot_bytes;
   a.lut_shift = batch.lut_shift;
   a.lut_bytes = batch.lut_bytes;
-  a.ring_offset = batch.item[ti].ring_offset;
   a.canon = batch.canon;
   a.out_bf16 = batch.item[ti].out_bf16;
   a.out_exp = batch.item[ti].out_exp;
@@ -881,7 +874,7 @@ decode_kernel(const BatchArgs batch) {
   const uint32_t slot0 = smem_u32(slots) + warp * bufs * buf_bytes;
   // per-warp ring for the packed fractions, behind all slots and their guard band
   const uint32_t ring =
-      smem_u32(smem) + a.ring_offset + warp * ring_warp_bytes(S) + lane * (S == 7 ? 8 : 4);
+      smem_u32(smem) + batch.item[ti].ring_offset + warp * ring_warp_bytes(S) + lane * (S == 7 ? 8 : 4);
 
   // Each warp owns one mbarrier; its lane 0 initialises it and is the only
   // thread that ever arms it.

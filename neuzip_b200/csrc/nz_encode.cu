@@ -1284,7 +1284,8 @@ place_units_kernel(const uint16_t *__restrict__ in, uint64_t n, uint32_t LS, uin
     const uint32_t *src = reinterpret_cast<const uint32_t *>(slots + (uint64_t)u * slot_stride);
     // 32-bit stores; when the destination starts on an odd word, one 16-bit store first and
     // then source words shifted by half a word.  The copy is bound by the latency of its
-    // loads: kBatch of them are in flight per lane.
+    // loads: kBatch of them are in flight per lane (4, 12 and 20: 77.4, 76.5 and 77.1 us for a
+    // compress of 4096 units of 256 symbols, 352, 346 and 355 for 28672).
     const uint32_t odd = w0 & 1u;
     if (odd && lane == 0) dst[0] = reinterpret_cast<const uint16_t *>(src)[0];
     uint32_t *d32 = reinterpret_cast<uint32_t *>(dst + odd);
@@ -1447,7 +1448,10 @@ static int compress_fused(const void *in, uint64_t n, uint32_t LS, uint32_t cols
     NZ_CUDA_TRY(launch_dependent(scan_kernel, 1, 1024, 0, st, (const uint32_t *)(sc + L.unit_words),
                                  nu, n, LS, (const uint32_t *)misc, cont));
   if (nu) {
-    // a unit per warp while that leaves blocks to spare, four on large tensors (less to add up)
+    // Units per block of the placement: one per warp, or four per warp on large tensors, whose
+    // blocks then add up fewer sizes in all.  Whole compress on a B200: 4096 units of 256 symbols
+    // 76.5 us with 4 and 82.5 with 16, 16384 units 210 and 213, 28672 units 346 and 348; 65536
+    // units of 8 symbols 98 and 89.
     const uint32_t per = nu <= 8192 ? 4 : 16;
     NZ_CUDA_TRY(launch_dependent(place_units_kernel<S>, (nu + per - 1) / per, 128, 0, st,
                                  (const uint16_t *)in, n, LS, nu, cols,

@@ -353,7 +353,7 @@ constexpr uint32_t kTmemSlot = 232;      // u32: tensor-memory base address
 constexpr uint32_t kAbortSlot = 236;     // u32: abort flag
 constexpr uint32_t kLastSlot = 240;      // u32: this CTA arrived last at its row tile's counter
 constexpr uint32_t kCumOff = 256;        // u16[257]
-constexpr uint32_t kFlagOff = 256 + 520; // u32[3]
+constexpr uint32_t kFlagOff = 256 + 520; // u32[4]
 
 template <int S>
 __global__ void __launch_bounds__(kLinThreads, 1)
@@ -367,7 +367,6 @@ linear_kernel(const LinearArgs p, const __grid_constant__ CUtensorMap x_map) {
 
   DecodeArgs a;
   a.container = p.container;
-  a.container_bytes = p.container_bytes;
   a.frac = p.frac;
   a.n = (uint64_t)p.rows * p.cols;
   a.S = p.S;
@@ -379,7 +378,6 @@ linear_kernel(const LinearArgs p, const __grid_constant__ CUtensorMap x_map) {
   a.slot_bytes = p.slot_bytes;
   a.lut_shift = p.lut_shift;
   a.lut_bytes = p.lut_bytes;
-  a.ring_offset = 0;
   a.canon = p.canon;
   a.out_bf16 = nullptr;
   a.out_exp = nullptr;
