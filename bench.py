@@ -49,7 +49,7 @@ UNIT = "GB/s"
 # DRAM traffic of one decode launch over a layer set (7 matrices, precision 7),
 # dram__bytes_read.sum + dram__bytes_write.sum from the ncu capture summarised in
 # profiles/decode_kernel_precision7_layer_set.md; scaled to the average launch by elements.
-NCU_TRAFFIC_BYTES = 271.26e6 + 347.1e6   # read (= the compressed bytes, no re-reads) + written
+NCU_TRAFFIC_BYTES = 317.24e6 + 348.55e6   # read (271.1e6 compressed bytes, some twice) + written
 # by kernel end; the rest of the 404.8 MB output is still in L2 then and is written back
 # while the next launch runs
 NCU_TRAFFIC_ELEMENTS = 4 * 4096 * 4096 + 3 * 4096 * 11008
