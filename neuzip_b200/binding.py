@@ -166,7 +166,10 @@ class Manager:
         """Let `linear` with at most `max_rows` input rows (tokens) decode the weight
         straight into tensor-core operand tiles instead of decompressing it first
         (0 switches it off).  Same fp32 accumulation as the library GEMM, different order
-        of the sums."""
+        of the sums.  Not faster at every shape: its work items (128 rows of the weight by one
+        unit) should make one wave on the SMs.  On a B200, fused against decompress and library
+        GEMM, 16 / 128 input rows: 4096 x 4096 22 / 27 against 28 / 29 us, 4096 x 11008 48 / 55
+        against 55 / 56, but 11008 x 4096 (three waves) 61 / 73 against 54 / 51."""
         if hasattr(self._be, "fused_linear_max_rows"):
             self._be.fused_linear_max_rows = int(max_rows)
 
