@@ -131,6 +131,9 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
     return !pairs_only && each <= max_warps &&
            (4096u << sh) + guard[t] + each * (b.item[t].slot_bytes + ring_bytes) <= sm_smem;
   };
+  bool hidden = true;          // every tensor's inputs are stable: the set-up overlaps the kernel before
+  for (uint32_t t = 0; t < count; ++t) hidden = hidden && (items[t].flags & NZ_ITEM_INPUTS_STABLE);
+  hidden = hidden || (precision == 7 && !items[0].out_exp);    // (exponent streams have 10 bits)
   const uint32_t pb = usual_prob_bits(precision);
   uint64_t best = ~0ull;
   uint32_t ctas[kMaxBatch] = {};
@@ -187,11 +190,15 @@ static int decode_geometry(const HostItem *items, uint32_t count, int precision,
         ++now[hi];
       }
     }
-    // the table has to be written first: 16 bytes per lane and store, by the few warps that a
-    // small launch has
+    // The table has to be written first, 16 bytes per lane and store.  A small launch has few warps
+    // for that, and it shows where the launch does not overlap the kernel before it (fresh inputs)
+    // and the table does not have the 32 copies whose stores are unrolled, as precision 7 does
+    // beside 64 KB.  Reads of 444 x 1600 and 512 x 1024 elements, one unit per CTA, in us beside 16
+    // and 64 KB: precision 7 overlapped 9.71, 9.22 and 6.93, 6.55, fresh 14.34, 13.19 and 11.53, 10.73;
+    // precision 3 overlapped 9.85, 9.54 and 7.04, 6.76, but fresh 16.3, 19.4 and 13.4, 16.8.
     uint64_t worst = 0;
     for (uint32_t t = 0; t < count; ++t) {
-      const uint32_t each = own(t, now[t]), writers = each < 4 ? each : 4;
+      const uint32_t each = own(t, now[t]), writers = each < 4 && !hidden ? each : 4;
       const uint64_t c = cost(t, now[t]) + (4096u << sh) / (16 * writers);
       if (c > worst) worst = c;
     }
